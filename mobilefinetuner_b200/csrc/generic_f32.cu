@@ -1,6 +1,7 @@
 // Generic fp32 kernels behind the eager `ops::` surface of the operator API:
-// broadcasting element-wise arithmetic, unary maps, reductions, permutes, a
-// batched fp32 matmul, row softmax, rotate-half RoPE on [B,H,S,D] tensors.
+// broadcasting element-wise arithmetic, unary maps, reductions, permutes,
+// row softmax, rotate-half RoPE on [B,H,S,D] tensors (the matrix product is in
+// matmul_f32.cu).
 // They exist so that every public operator of the reference works on
 // device-resident tensors with fp32 accuracy (its own unit tests hold 1e-5 ..
 // 1e-6); the fused bf16 tensor-core kernels are what the training step uses.
@@ -98,30 +99,6 @@ __global__ void permute_kernel(const uint32_t* __restrict__ in, uint32_t* __rest
         }
         out[i] = in[src];
     }
-}
-
-// C[b] (M x N) = A[b] (M x K) * op(B[b]) ; B is [K,N] (trans_b = 0) or [N,K] (trans_b = 1); fp32 FMA, 32x32 tiles.
-__global__ void matmul_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C, int M, int N, int K,
-                                  int64_t stride_a, int64_t stride_b, int64_t stride_c, int trans_b) {
-    __shared__ float As[32][33], Bs[32][33];
-    const int b = blockIdx.z;
-    const float* a = A + b * stride_a;
-    const float* bb = B + b * stride_b;
-    float* c = C + b * stride_c;
-    const int row = blockIdx.y * 32 + threadIdx.y, col = blockIdx.x * 32 + threadIdx.x;
-    float acc = 0.f;
-    for (int k0 = 0; k0 < K; k0 += 32) {
-        const int ka = k0 + threadIdx.x, kb = k0 + threadIdx.y;
-        As[threadIdx.y][threadIdx.x] = (row < M && ka < K) ? a[(int64_t)row * K + ka] : 0.f;
-        float bv = 0.f;
-        if (kb < K && col < N) bv = trans_b ? bb[(int64_t)col * K + kb] : bb[(int64_t)kb * N + col];
-        Bs[threadIdx.y][threadIdx.x] = bv;
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < 32; ++k) acc = fmaf(As[threadIdx.y][k], Bs[k][threadIdx.x], acc);
-        __syncthreads();
-    }
-    if (row < M && col < N) c[(int64_t)row * N + col] = acc;
 }
 
 __global__ void softmax_fwd_kernel(const float* __restrict__ x, float* __restrict__ y, int64_t dim) {
@@ -258,16 +235,6 @@ int32_t mft_permute_b32(const void* in, void* out, const int64_t* in_shape, cons
     if (n == 0) return MFT_OK;
     permute_kernel<<<grid1(n), 256, 0, as_stream(stream)>>>((const uint32_t*)in, (uint32_t*)out, n, p);
     MFT_LAUNCH_CHECK("permute_b32");
-    return MFT_OK;
-}
-
-int32_t mft_matmul_f32(const float* a, const float* b, float* c, int64_t batch, int64_t m, int64_t n, int64_t k, int64_t stride_a,
-                       int64_t stride_b, int64_t stride_c, int32_t trans_b, mft_stream_t stream) {
-    MFT_CHECK_ARG(a && b && c && batch > 0 && m > 0 && n > 0 && k > 0 && batch <= 65535, "mft_matmul_f32: bad argument");
-    dim3 grid((unsigned)((n + 31) / 32), (unsigned)((m + 31) / 32), (unsigned)batch);
-    MFT_CHECK_ARG(grid.y <= 65535, "mft_matmul_f32: M too large");
-    matmul_f32_kernel<<<grid, dim3(32, 32), 0, as_stream(stream)>>>(a, b, c, (int)m, (int)n, (int)k, stride_a, stride_b, stride_c, trans_b);
-    MFT_LAUNCH_CHECK("matmul_f32");
     return MFT_OK;
 }
 
