@@ -121,40 +121,43 @@ gemm_nt_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            int stage = 0; uint32_t phase = 0;
-            int it = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++it) {
-                const int acc = it & 1;
-                const uint32_t acc_phase = (it >> 1) & 1;
-                if (!mbar_wait(&tmem_empty_bar[acc], acc_phase ^ 1, abort_flag)) { ok = false; break; }
+        // ------------------------------------------------ MMA issuer (warp-uniform loop, one elected lane issues: see the pair kernel)
+        int stage = 0; uint32_t phase = 0;
+        int it = 0;
+        bool ok = true;
+        const uint64_t desc0 = smem_desc_sw128(smem_u32(tiles));
+        auto wait_all = [&](uint64_t* bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)) != 0; };
+        for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++it) {
+            const int acc = it & 1;
+            const uint32_t acc_phase = (it >> 1) & 1;
+            if (!wait_all(&tmem_empty_bar[acc], acc_phase ^ 1)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t tmem_d = tmem_base + acc * BN;
+            const int split = tile / p.tiles_mn;
+            const int kb0 = split * p.kb_per_split, kb1 = min(num_kb, kb0 + p.kb_per_split);
+            // a ragged last column tile issues narrower MMAs (existing columns rounded up to 16)
+            const int n_left = p.n - tile_n(tile % p.tiles_mn, p) * BN;
+            const uint32_t idesc = idesc_bf16_f32(GEMM_BM, (uint32_t)min(BN, (n_left + 15) & ~15));
+            for (int kb = kb0; kb < kb1; ++kb) {
+                if (!wait_all(&full_bar[stage], phase)) { ok = false; break; }
                 tc_fence_after();
-                const uint32_t tmem_d = tmem_base + acc * BN;
-                const int split = tile / p.tiles_mn;
-                const int kb0 = split * p.kb_per_split, kb1 = min(num_kb, kb0 + p.kb_per_split);
-                // a ragged last column tile issues narrower MMAs (existing columns rounded up to 16)
-                const int n_left = p.n - tile_n(tile % p.tiles_mn, p) * BN;
-                const uint32_t idesc = idesc_bf16_f32(GEMM_BM, (uint32_t)min(BN, (n_left + 15) & ~15));
-                for (int kb = kb0; kb < kb1; ++kb) {
-                    if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t sa = smem_u32(tiles + stage * Cfg::STAGE_BYTES);
-                    const uint32_t sb = sa + Cfg::A_BYTES;
-                    const uint64_t adesc = smem_desc_sw128(sa);
-                    const uint64_t bdesc = smem_desc_sw128(sb);
-                    const int kvalid = (kb < num_kb_main) ? min(GEMM_BK, p.k - kb * GEMM_BK) : p.k2;
-                    const int nmma = (kvalid + 15) / 16;
-                    for (int j = 0; j < nmma; ++j) {
-                        // advance 16 bf16 = 32 bytes along K inside the swizzle atom: +2 in 16-byte units
-                        umma_bf16(tmem_d, adesc + (uint64_t)(2 * j), bdesc + (uint64_t)(2 * j), idesc, (kb > kb0 || j != 0) ? 1u : 0u);
+                const uint64_t adesc = desc0 + (uint64_t)(stage * (Cfg::STAGE_BYTES >> 4)), bdesc = adesc + (Cfg::A_BYTES >> 4);
+                const int nmma = ((kb < num_kb_main ? min(GEMM_BK, p.k - kb * GEMM_BK) : p.k2) + 15) / 16;
+                if (elect_one()) {
+                    // 16 bf16 = 32 bytes along K inside the swizzle atom: +2 in 16-byte units
+                    if (nmma == 4) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) umma_bf16(tmem_d, adesc + 2 * j, bdesc + 2 * j, idesc, (kb > kb0 || j != 0) ? 1u : 0u);
+                    } else {
+                        for (int j = 0; j < nmma; ++j) umma_bf16(tmem_d, adesc + 2 * j, bdesc + 2 * j, idesc, (kb > kb0 || j != 0) ? 1u : 0u);
                     }
                     umma_commit(&empty_bar[stage]);   // frees the stage once these MMAs have read it
-                    if (++stage == Cfg::STAGES) { stage = 0; phase ^= 1; }
                 }
-                if (ok) umma_commit(&tmem_full_bar[acc]);
+                __syncwarp();
+                if (++stage == Cfg::STAGES) { stage = 0; phase ^= 1; }
             }
+            if (ok && elect_one()) umma_commit(&tmem_full_bar[acc]);
+            __syncwarp();
         }
     } else {
         // ------------------------------------------------ epilogue (warps 2..5)
