@@ -98,6 +98,10 @@ __device__ __forceinline__ uint64_t smem_desc_mn_sw128(uint32_t smem_addr, uint3
     d |= (uint64_t)2 << 61;
     return d;
 }
+// Wait of a whole MMA-issuing warp: the warp stays converged, one elected lane issues (see the pair GEMM's issuer)
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)) != 0;
+}
 constexpr uint32_t IDESC_B_MN = 1u << 16;      // instruction-descriptor bit: B operand is MN-major
 
 struct FwdParams {
@@ -209,15 +213,16 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         // (The tensor pipe takes MMAs from a thread only about as fast as that thread issues them: every wait,
         // fence and commit between two MMAs is exposed when the MMAs are short.  Two issuing threads overlap
         // one product's bookkeeping with the other product's MMAs.)
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc_s = idesc_bf16_f32(BM, BN);
-            bool ok = mbar_wait(q_full, 0, abort_flag);
+            bool ok = warp_wait(q_full, 0, abort_flag);
             const uint64_t qd = smem_desc_sw128(smem_u32(q_smem));
             for (int t = 0; t < n_tiles && ok; ++t) {
                 const int st = t & 1;
                 const uint32_t ph = (t >> 1) & 1;
-                if (!mbar_wait(&k_full[st], ph, abort_flag) || !mbar_wait(&s_free[st], ph ^ 1, abort_flag)) { ok = false; break; }
+                if (!warp_wait(&k_full[st], ph, abort_flag) || !warp_wait(&s_free[st], ph ^ 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
+                if (elect_one()) {
                 const uint64_t kd = smem_desc_sw128(smem_u32(k_smem + st * KV_BYTES));
                 const uint32_t tmem_s = tmem_base + S_COL + st * BN;
 #pragma unroll
@@ -228,11 +233,13 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                                   (c | j) != 0 ? 1u : 0u);
                 umma_commit(&k_empty[st]);
                 umma_commit(&s_full[st]);
+                }
+                __syncwarp();
             }
         }
     } else if (warp == 10) {
         // ------------------------------------------------ MMA issuer 2: O += P V
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc_o = idesc_bf16_f32(BM, HD) | IDESC_B_MN;
             bool ok = true;
             int vs = 0;
@@ -240,8 +247,9 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             for (int t = 0; t < n_tiles && ok; ++t) {
                 const int st = t & 1;
                 const uint32_t ph = (t >> 1) & 1;
-                if (!mbar_wait(&v_full[vs], vph, abort_flag) || !mbar_wait(&p_full[st], ph, abort_flag)) { ok = false; break; }
+                if (!warp_wait(&v_full[vs], vph, abort_flag) || !warp_wait(&p_full[st], ph, abort_flag)) { ok = false; break; }
                 tc_fence_after();
+                if (elect_one()) {
                 // A = the bf16 probabilities in tensor memory (8 columns per 16 keys), B = V as it lies in memory
                 const uint32_t pa = tmem_base + P_COL + st * 32;
                 const uint64_t vd = smem_desc_mn_sw128(smem_u32(v_smem + vs * KV_BYTES), BN * 128);
@@ -251,6 +259,8 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 umma_commit(&v_empty[vs]);
                 umma_commit(&p_free[st]);
                 umma_commit(&o_done[st]);
+                }
+                __syncwarp();
                 if (++vs == FWD_VST) { vs = 0; vph ^= 1; }
             }
         }
@@ -495,17 +505,18 @@ attn_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         }
     } else if (warp == 1 || warp == W_DP) {
         // ------------------------------------------------ MMA issuers 1 and 2: S = Q K^T (warp 1), dP = dO V^T (warp W_DP)
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc_s = idesc_bf16_f32(BM, DQ_BN);
             const bool is_s = warp == 1;
-            bool ok = mbar_wait(qdo_full, 0, abort_flag);
+            bool ok = warp_wait(qdo_full, 0, abort_flag);
             const uint64_t ad = smem_desc_sw128(smem_u32(is_s ? q_smem : do_smem));
             for (int t = 0; t < n_tiles && ok; ++t) {
                 const int g = t & 1, ks = t % DQ_KST;
                 const uint32_t gph = (t >> 1) & 1, kph = (t / DQ_KST) & 1;
-                if (is_s ? !mbar_wait(&k_full[ks], kph, abort_flag) : !mbar_wait(&v_full[g], gph, abort_flag)) { ok = false; break; }
-                if (!mbar_wait(&sdp_free[g], gph ^ 1, abort_flag)) { ok = false; break; }
+                if (!warp_wait(is_s ? &k_full[ks] : &v_full[g], is_s ? kph : gph, abort_flag)) { ok = false; break; }
+                if (!warp_wait(&sdp_free[g], gph ^ 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
+                if (elect_one()) {
                 const uint64_t bd = smem_desc_sw128(smem_u32(is_s ? k_smem + ks * DQ_KV_BYTES : v_smem + g * DQ_KV_BYTES));
                 const uint32_t tmem_d = tmem_base + (is_s ? DQ_S_COL : DQ_DP_COL) + g * DQ_BN;
 #pragma unroll
@@ -516,18 +527,21 @@ attn_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                                   (c | j) != 0 ? 1u : 0u);
                 if (!is_s) umma_commit(&v_empty[g]);
                 umma_commit(&sdp_full[g]);            // two arrivals complete it: S and dP
+                }
+                __syncwarp();
             }
         }
     } else if (warp == W_DQ) {
         // ------------------------------------------------ MMA issuer 3: dQ += dS K
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc_acc = idesc_bf16_f32(BM, HD) | IDESC_B_MN;
             bool ok = true;
             for (int t = 0; t < n_tiles && ok; ++t) {
                 const int g = t & 1, ks = t % DQ_KST;
                 const uint32_t gph = (t >> 1) & 1;
-                if (!mbar_wait(&ds_full[g], gph, abort_flag)) { ok = false; break; }
+                if (!warp_wait(&ds_full[g], gph, abort_flag)) { ok = false; break; }
                 tc_fence_after();
+                if (elect_one()) {
                 const uint64_t kd = smem_desc_mn_sw128(smem_u32(k_smem + ks * DQ_KV_BYTES), DQ_BN * 128);
 #pragma unroll
                 for (int j = 0; j < 2; ++j)
@@ -535,6 +549,8 @@ attn_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                 umma_commit(&k_empty[ks]);
                 umma_commit(&ds_free[g]);
                 if (t == n_tiles - 1) umma_commit(acc_done);
+                }
+                __syncwarp();
             }
         }
     } else {
@@ -755,10 +771,10 @@ attn_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         }
     } else if (warp == 1 || warp == W_DP) {
         // ------------------------------------------------ MMA issuers 1 and 2: S^T = K Q^T (warp 1), dP^T = V dO^T (warp W_DP)
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc_s = idesc_bf16_f32(BM, KV_BQ);
             const bool is_s = warp == 1;
-            bool ok = mbar_wait(kv_full, 0, abort_flag);
+            bool ok = warp_wait(kv_full, 0, abort_flag);
             const uint64_t ad = smem_desc_sw128(smem_u32(is_s ? k_smem : v_smem));
             int st = 0;
             uint32_t sph = 0;
@@ -766,8 +782,9 @@ attn_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 const int g = t & 1;
                 const uint32_t ph = (t >> 1) & 1;
                 // in place: the buffer also holds P^T / dS^T of tile t - 2 until that tile's dV / dK products are done
-                if (!mbar_wait(&qdo_full[st], sph, abort_flag) || !mbar_wait(INPLACE ? &pds_free[g] : &sdp_free[g], ph ^ 1, abort_flag)) { ok = false; break; }
+                if (!warp_wait(&qdo_full[st], sph, abort_flag) || !warp_wait(INPLACE ? &pds_free[g] : &sdp_free[g], ph ^ 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
+                if (elect_one()) {
                 const uint64_t bd = smem_desc_sw128(smem_u32((is_s ? q_smem : do_smem) + st * KV_Q_BYTES));
                 const uint32_t tmem_d = tmem_base + (is_s ? KV_S_COL : KV_DP_COL) + g * KV_BQ;
 #pragma unroll
@@ -777,20 +794,23 @@ attn_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                         umma_bf16(tmem_d, ad + (uint64_t)(c * (BM * 128 / 16) + 2 * j), bd + (uint64_t)(c * (KV_BQ * 128 / 16) + 2 * j), idesc_s,
                                   (c | j) != 0 ? 1u : 0u);
                 umma_commit(&sdp_full[g]);
+                }
+                __syncwarp();
                 if (++st == KV_STAGES) { st = 0; sph ^= 1; }
             }
         }
     } else if (warp == W_ACC) {
         // ------------------------------------------------ MMA issuer 3: dV += P^T dO, dK += dS^T Q (this CTA's 128 columns)
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc_acc = idesc_bf16_f32(BM, ACC) | IDESC_B_MN;
             bool ok = true;
             int st = 0;
             for (int t = 0; t < n_tiles && ok; ++t) {
                 const int g = t & 1;
                 const uint32_t ph = (t >> 1) & 1;
-                if (!mbar_wait(&pds_full[g], ph, abort_flag)) { ok = false; break; }
+                if (!warp_wait(&pds_full[g], ph, abort_flag)) { ok = false; break; }
                 tc_fence_after();
+                if (elect_one()) {
                 // A operands P^T / dS^T come from tensor memory (8 columns per 16 queries), B operands dO / Q MN-major from the stage
                 // separate: P^T at pa + {0, 8}, dS^T at pa + 16 + {0, 8}.  In place: P^T in the S^T buffer at +{0, 16}
                 // (the first 8 columns of each half's 16), dS^T in the dP^T buffer likewise
@@ -808,6 +828,8 @@ attn_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 umma_commit(&qdo_empty[st]);
                 umma_commit(&pds_free[g]);
                 if (t == n_tiles - 1) umma_commit(acc_done);
+                }
+                __syncwarp();
                 if (++st == KV_STAGES) st = 0;
             }
         }
