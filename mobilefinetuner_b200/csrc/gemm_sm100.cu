@@ -484,6 +484,8 @@ static int32_t gemm_nt_run_inner(const GemmCall& c, cudaStream_t stream) {
     // CTA-pair kernel first (256 x 256 cluster tiles); MFT_GEMM_2CTA=0 selects the single-CTA kernel everywhere
     static const int use_pair = [] { const char* e = std::getenv("MFT_GEMM_2CTA"); return e ? std::atoi(e) : 1; }();
     if (use_pair && device_status_word()) {
+        const int32_t s1 = gemm_nt_run_ksplit(c, stream);
+        if (s1 != MFT_ERR_UNSUPPORTED) return s1;
         const int32_t s2 = gemm_nt_run_2cta(c, stream);
         if (s2 != MFT_ERR_UNSUPPORTED) return s2;
     }

@@ -92,6 +92,11 @@ __host__ __device__ inline int tile_n(int tile, const GemmParams& p) {
 int32_t gemm_nt_run(const GemmCall& c, cudaStream_t stream);
 // CTA-pair (cta_group::2) variant for 256 x 256 cluster tiles; returns MFT_ERR_UNSUPPORTED when the call does not qualify.
 int32_t gemm_nt_run_2cta(const GemmCall& c, cudaStream_t stream);
+// K-split variant for bf16 outputs of few tiles (gemm_ksplit.cu); MFT_ERR_UNSUPPORTED when the call does not qualify or
+// another kernel is the faster one.
+struct KsplitPlan { int bn = 0, splits = 1; };
+KsplitPlan ksplit_plan(int64_t m, int64_t n, int64_t k, int64_t k2);
+int32_t gemm_nt_run_ksplit(const GemmCall& c, cudaStream_t stream);
 // columns of the pair kernel's tile for a plain-store call of this shape: 256, 384 (long K under a width that is a
 // multiple of 384), or 0 when the pair kernel does not take the call
 int gemm_nt_pair_tile_cols(int64_t m, int64_t n, int64_t k, int64_t k2, bool d_is_f32);

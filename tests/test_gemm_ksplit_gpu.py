@@ -1,0 +1,36 @@
+"""bf16 GEMM with K cut over the CTAs of a cluster, at the edges of its tiles, k-blocks and K ranges, against float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+BF = torch.bfloat16
+
+
+@pytest.mark.parametrize("m,n,k,k2,bias", [
+    (512, 16, 13824, 0, False), (512, 48, 1152, 0, False), (130, 40, 520, 0, False), (512, 1152, 13824, 32, False), (512, 1536, 1152, 48, False), (1, 64, 704, 0, False),
+    (129, 72, 1352, 16, True), (437, 640, 2048, 8, False), (437, 8, 640, 0, False), (512, 2304, 768, 8, True), (65, 128, 1000, 0, True),
+    (1985, 896, 4864, 0, False), (300, 200, 1160, 64, True), (512, 50, 6912, 0, True), (1000, 768, 3072, 0, False)])
+def test_gemm_ksplit(m, n, k, k2, bias):
+    from mobilefinetuner_b200 import ops as O
+    g = torch.Generator(device="cuda").manual_seed(m * 131 + n * 7 + k)
+
+    def rnd(r, c, scale=1.0):
+        return (torch.randn(r, c, device="cuda", generator=g) * scale).to(BF)
+    a, b = rnd(m, k), rnd(n, k, 0.05)
+    a2, b2 = (rnd(m, 64)[:, :k2], rnd(n, 64, 0.05)[:, :k2]) if k2 else (None, None)
+    if k2 % 16:      # the second segment's columns up to the next multiple of 16 take part: zero, as the rank panels are
+        a2, b2 = torch.zeros(m, 64, device="cuda", dtype=BF), torch.zeros(n, 64, device="cuda", dtype=BF)
+        a2[:, :k2], b2[:, :k2] = rnd(m, k2), rnd(n, k2, 0.05)
+        a2, b2 = a2[:, :k2], b2[:, :k2]
+    bs = torch.randn(n, device="cuda", generator=g) if bias else None
+    ld = (n + 7) // 8 * 8
+    out = torch.full((m + 1, ld), 7.0, device="cuda", dtype=BF)
+    O.gemm_nt(a, b, a2=a2, b2=b2, bias=bs, alpha=0.5, out=out[:m, :n])
+    want, mag = a.double() @ b.double().T, a.double().abs() @ b.double().abs().T
+    if k2:
+        want, mag = want + a2.double() @ b2.double().T, mag + a2.double().abs() @ b2.double().abs().T
+    want = 0.5 * want + (bs.double() if bias else 0.0)
+    # bf16 rounding of the result (2^-9 relative) and the f32 sums of k + k2 exact products, alpha, bias and the slices
+    bound = 2.0 ** -8 * want.abs() + (k + k2 + 16) * 2.0 ** -24 * (mag + 1.0)
+    assert bool(((out[:m, :n].double() - want).abs() <= bound).all())
+    assert bool((out[m] == 7.0).all()) and bool((out[:m, n:] == 7.0).all())
