@@ -114,14 +114,16 @@ int32_t refresh_panels(mft_model* m) {
     return MFT_OK;
 }
 
-int32_t forward(Ctx& c, bool for_training, int64_t n_valid_global = 0) {
+// What follows the final norm: nothing (the caller goes on from m->hf), the loss, or the loss with d(loss)/d(hidden).
+enum class Head { kNone, kLoss, kTrain };
+
+int32_t forward(Ctx& c, Head head, int64_t n_valid_global = 0) {
     mft_model* m = c.m;
     const mft_model_config_t& cfg = m->cfg;
     const bool gpt2 = cfg.family == MFT_FAMILY_GPT2, gemma = cfg.family == MFT_FAMILY_GEMMA;
     const int H = cfg.hidden, I = cfg.inter, nh = cfg.n_heads, nkv = cfg.n_kv_heads, hd = cfg.head_dim, L = cfg.layers;
     const int QD = nh * hd, KD = nkv * hd, QKV = QD + 2 * KD;
     const int64_t T = c.T, S = c.S;
-    (void)for_training;
     const bool fuse = gemma && m->fuse_norms && H <= 2048;      // Gemma's post-norm + residual + pre-norm pairs in one kernel
     TRY(mft_memset(m->status_dev, 0, 4, c.st));
     const float emb_scale = gemma ? std::sqrt((float)H) : 1.0f;
@@ -181,9 +183,12 @@ int32_t forward(Ctx& c, bool for_training, int64_t n_valid_global = 0) {
     }
     if (gpt2) TRY(mft_layernorm_fwd(m->x_final, MFT_F32, m->final_w, m->final_b, 1e-5f, m->hf, MFT_BF16, m->mean_f, m->rstd_f, T, H, c.st));
     else if (!fuse) TRY(mft_rmsnorm_fwd(m->x_final, MFT_F32, m->final_w, cfg.norm_eps, gemma ? 1 : 0, m->hf, MFT_BF16, m->rstd_f, nullptr, nullptr, T, H, c.st));
+    // callers that only want the final hidden states (their token ids were checked by the embedding): the loss sweep would
+    // read the whole vocabulary table against every position for nothing
+    if (head == Head::kNone) return MFT_OK;
     // lm head + shifted cross entropy; the [T,V] logits are never written.  A training step gets the loss and
     // d(loss)/d(final hidden) (into t_h) from one sweep over the vocabulary.
-    if (for_training && m->ce_onepass)
+    if (head == Head::kTrain && m->ce_onepass)
         return mft_lmhead_ce_fused(m->hf, m->embed, m->embed_t, m->ld_t, m->labels, c.B, S, H, cfg.vocab, -100, n_valid_global, m->loss_scale,
                                    m->loss_dev, m->n_valid_dev, m->ce_lse, m->t_h, m->status_dev, m->ce_ws, m->ce_ws_bytes, c.st);
     return mft_lmhead_ce_fwd(m->hf, m->embed, m->labels, c.B, S, H, cfg.vocab, -100, m->loss_dev, m->n_valid_dev, m->ce_lse, m->status_dev,
@@ -303,7 +308,7 @@ int32_t forward_backward(Ctx& c, int64_t n_valid_global) {
     if (m->merged) return fail(MFT_ERR_INVALID_ARG, "the adapters are merged into the base weights: call mft_model_unmerge_lora before training");
     TRY(refresh_panels(m));
     auto eager = [&]() -> int32_t {
-        TRY(forward(c, true, n_valid_global));
+        TRY(forward(c, Head::kTrain, n_valid_global));
         return backward(c, n_valid_global);
     };
     if (!m->use_graph || gemm_profiling_enabled()) return eager();
@@ -336,7 +341,7 @@ int32_t forward_backward(Ctx& c, int64_t n_valid_global) {
             return eager();
         }
         const int64_t launches_before = mft_launch_count();
-        int32_t s = forward(cc, true, n_valid_global);
+        int32_t s = forward(cc, Head::kTrain, n_valid_global);
         if (s == MFT_OK) s = backward(cc, n_valid_global);
         g->kernels = mft_launch_count() - launches_before;
         count_launch(-(int)g->kernels);                      // captured, not run: counted at every replay instead
@@ -395,7 +400,7 @@ extern "C" int32_t mft_model_forward_loss(mft_model_t* m, const int32_t* ids_hos
     TRY(mft_memcpy_h2d(m->ids, ids_host, (size_t)c.T * 4, c.st));
     TRY(mft_memcpy_h2d(m->labels, labels_host, (size_t)c.T * 4, c.st));
     TRY(refresh_panels(m));
-    TRY(forward(c, false));
+    TRY(forward(c, Head::kLoss));
     TRY(mft_memcpy_d2h(loss_host, m->loss_dev, 4, c.st));
     return check_status(m);
 }
@@ -408,9 +413,8 @@ extern "C" int32_t mft_model_forward_logits(mft_model_t* m, const int32_t* ids_h
     TRY(make_ctx(m, batch, seq, &c));
     MFT_CHECK_ARG(ids_host && logits_dev, "mft_model_forward_logits: null argument");
     TRY(mft_memcpy_h2d(m->ids, ids_host, (size_t)c.T * 4, c.st));
-    TRY(mft_memcpy_h2d(m->labels, ids_host, (size_t)c.T * 4, c.st));      // any valid labels: the loss is not used
     TRY(refresh_panels(m));
-    TRY(forward(c, false));
+    TRY(forward(c, Head::kNone));
     TRY(mft_gemm_nt(m->hf, m->cfg.hidden, m->embed, m->cfg.hidden, c.T, m->cfg.vocab, m->cfg.hidden, nullptr, 0, nullptr, 0, 0, nullptr, 1.0f,
                     logits_dev, m->cfg.vocab, MFT_F32, 0, c.st));
     return check_status(m);
@@ -422,9 +426,8 @@ extern "C" int32_t mft_model_forward_hidden(mft_model_t* m, const int32_t* ids_h
     TRY(make_ctx(m, batch, seq, &c));
     MFT_CHECK_ARG(ids_host && hidden_dev, "mft_model_forward_hidden: null argument");
     TRY(mft_memcpy_h2d(m->ids, ids_host, (size_t)c.T * 4, c.st));
-    TRY(mft_memcpy_h2d(m->labels, ids_host, (size_t)c.T * 4, c.st));
     TRY(refresh_panels(m));
-    TRY(forward(c, false));
+    TRY(forward(c, Head::kNone));
     TRY(mft_cast_bf16_to_f32(m->hf, hidden_dev, c.T * m->cfg.hidden, c.st));
     return check_status(m);
 }
@@ -512,9 +515,8 @@ extern "C" int32_t mft_model_score_tokens(mft_model_t* m, const int32_t* ids_hos
     TRY(make_ctx(m, 1, seq, &c));
     const int64_t H = m->cfg.hidden, V = m->cfg.vocab;
     TRY(mft_memcpy_h2d(m->ids, ids_host, (size_t)seq * 4, c.st));
-    TRY(mft_memcpy_h2d(m->labels, ids_host, (size_t)seq * 4, c.st));      // any valid labels: the loss is not used
     TRY(refresh_panels(m));
-    TRY(forward(c, false));
+    TRY(forward(c, Head::kNone));
     // scratch inside the staging buffer: candidate rows (f32, then bf16), the last hidden row twice, logits, ids
     MFT_CHECK_ARG((64 + 2) * H * 2 + 1024 <= m->stage_floats - 64, "mft_model_score_tokens: staging buffer too small");
     float* rows_f32 = m->stage_f32;
