@@ -17,8 +17,8 @@ struct AttnParams {
     int window;
 };
 
-// Forward pass on the 5th-generation tensor cores (head_dim 256, sequence a multiple of 128, token-major
-// operands).  Returns MFT_ERR_UNSUPPORTED when the problem does not qualify; the caller then uses the
+// Forward pass on the 5th-generation tensor cores (head_dim 64, 128 or 256, any sequence length above a measured one,
+// token-major operands).  Returns MFT_ERR_UNSUPPORTED when the problem does not qualify; the caller then uses the
 // mma.sync kernel.
 int32_t attn_fwd_sm100(const AttnParams& p, int hd, cudaStream_t stream);
 // dQ of the backward pass, same conditions.  With compute_delta the kernel also forms delta = rowsum(O * dO) and

@@ -14,6 +14,10 @@
 // V is consumed as it lies in memory ([key][d], "MN-major" B operand), so nothing is transposed.
 // The reference maximum is only raised (and O rescaled in tensor memory) when a row's maximum grew by more
 // than 2^8 since the last rescale, which keeps the exponentials below 256 and makes rescales rare.
+// Sequences of any length: the tensor maps are [batch, sequence, columns], so that a tile's rows past the end of a sequence
+// read as zeros (never as the next sample), and only stores look at the length; the causal mask hides keys past the end from
+// every row that is stored.  At 3 x 1001 tokens, 4 / 1 heads of 256, forward / dQ / dK + dV took 54 / 89 / 87 us on the
+// mma.sync kernels; the whole backward is 125 instead of 274 us at 4 x 1001.
 // Every mbarrier wait is bounded; a wait that runs out sets the library status word and the CTA leaves.
 #include <cuda.h>
 
@@ -164,7 +168,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     const int h = blockIdx.y, b = blockIdx.z;
     const int kvh = h / p.rep;
     const int i0 = qb * BM;
-    const int jb_hi = (i0 + BM - 1) / BN;
+    const int jb_hi = (min(i0 + BM, p.seq) - 1) / BN;
     const int jb_lo = p.window > 0 ? max(0, i0 - p.window + 1) / BN : 0;
     const int n_tiles = jb_hi - jb_lo + 1;
 
@@ -192,19 +196,19 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         if (lane == 0) {
             const int qx = h * p.q_col0_stride, kx = kvh * p.kv_col0_stride;
             mbar_arrive_expect_tx(q_full, Q_BYTES);
-            for (int c = 0; c < CH; ++c) tma_load_2d(q_smem + c * (BM * 128), &map_q, q_full, qx + c * 64, b * p.seq + i0);
+            for (int c = 0; c < CH; ++c) tma_load_3d(q_smem + c * (BM * 128), &map_q, q_full, qx + c * 64, i0, b);
             int vs = 0;
             uint32_t vph = 0;                           // V stage of tile t and its phase parity
             for (int t = 0; t < n_tiles; ++t) {
                 const int st = t & 1;
                 const uint32_t ph = (t >> 1) & 1;
-                const int row = b * p.seq + (jb_lo + t) * BN;
+                const int row = (jb_lo + t) * BN;
                 if (!mbar_wait(&k_empty[st], ph ^ 1, abort_flag)) break;
                 mbar_arrive_expect_tx(&k_full[st], KV_BYTES);
-                for (int c = 0; c < CH; ++c) tma_load_2d(k_smem + st * KV_BYTES + c * (BN * 128), &map_k, &k_full[st], kx + c * 64, row);
+                for (int c = 0; c < CH; ++c) tma_load_3d(k_smem + st * KV_BYTES + c * (BN * 128), &map_k, &k_full[st], kx + c * 64, row, b);
                 if (!mbar_wait(&v_empty[vs], vph ^ 1, abort_flag)) break;
                 mbar_arrive_expect_tx(&v_full[vs], KV_BYTES);
-                for (int c = 0; c < CH; ++c) tma_load_2d(v_smem + vs * KV_BYTES + c * (BN * 128), &map_v, &v_full[vs], kx + c * 64, row);
+                for (int c = 0; c < CH; ++c) tma_load_3d(v_smem + vs * KV_BYTES + c * (BN * 128), &map_v, &v_full[vs], kx + c * 64, row, b);
                 if (++vs == FWD_VST) { vs = 0; vph ^= 1; }
             }
         }
@@ -368,10 +372,10 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                     float t8[8];
 #pragma unroll
                     for (int e = 0; e < 8; ++e) t8[e] = __uint_as_float(o[x + e]) * inv;
-                    store8(orow + c + x, t8);
+                    if (i < p.seq) store8(orow + c + x, t8);
                 }
             }
-            if (half == 0) p.lse[((long long)b * p.n_heads + h) * p.seq + i] = (m_used + log2f(l)) / LOG2E;
+            if (half == 0 && i < p.seq) p.lse[((long long)b * p.n_heads + h) * p.seq + i] = (m_used + log2f(l)) / LOG2E;
         }
     }
 
@@ -463,7 +467,7 @@ attn_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     const int h = blockIdx.y, b = blockIdx.z;
     const int kvh = h / p.rep;
     const int i0 = qb * BM;
-    const int jb_hi = (i0 + BM - 1) / DQ_BN;
+    const int jb_hi = (min(i0 + BM, p.seq) - 1) / DQ_BN;
     const int jb_lo = p.window > 0 ? max(0, i0 - p.window + 1) / DQ_BN : 0;
     const int n_tiles = jb_hi - jb_lo + 1;
 
@@ -489,18 +493,18 @@ attn_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     if (warp == 0) {
         if (lane == 0) {
             mbar_arrive_expect_tx(qdo_full, 2 * Q_BYTES);
-            for (int c = 0; c < CH; ++c) tma_load_2d(q_smem + c * (BM * 128), &map_q, qdo_full, h * p.q_col0_stride + c * 64, b * p.seq + i0);
-            for (int c = 0; c < CH; ++c) tma_load_2d(do_smem + c * (BM * 128), &map_do, qdo_full, h * p.do_col0_stride + c * 64, b * p.seq + i0);
+            for (int c = 0; c < CH; ++c) tma_load_3d(q_smem + c * (BM * 128), &map_q, qdo_full, h * p.q_col0_stride + c * 64, i0, b);
+            for (int c = 0; c < CH; ++c) tma_load_3d(do_smem + c * (BM * 128), &map_do, qdo_full, h * p.do_col0_stride + c * 64, i0, b);
             for (int t = 0; t < n_tiles; ++t) {
                 const int ks = t % DQ_KST, vs = t & 1;
                 const uint32_t kph = (t / DQ_KST) & 1, vph = (t >> 1) & 1;
-                const int row = b * p.seq + (jb_lo + t) * DQ_BN;
+                const int row = (jb_lo + t) * DQ_BN;
                 if (!mbar_wait(&k_empty[ks], kph ^ 1, abort_flag)) break;
                 mbar_arrive_expect_tx(&k_full[ks], DQ_KV_BYTES);
-                for (int c = 0; c < CH; ++c) tma_load_2d(k_smem + ks * DQ_KV_BYTES + c * (DQ_BN * 128), &map_k, &k_full[ks], kvh * p.k_col0_stride + c * 64, row);
+                for (int c = 0; c < CH; ++c) tma_load_3d(k_smem + ks * DQ_KV_BYTES + c * (DQ_BN * 128), &map_k, &k_full[ks], kvh * p.k_col0_stride + c * 64, row, b);
                 if (!mbar_wait(&v_empty[vs], vph ^ 1, abort_flag)) break;
                 mbar_arrive_expect_tx(&v_full[vs], DQ_KV_BYTES);
-                for (int c = 0; c < CH; ++c) tma_load_2d(v_smem + vs * DQ_KV_BYTES + c * (DQ_BN * 128), &map_v, &v_full[vs], kvh * p.v_col0_stride + c * 64, row);
+                for (int c = 0; c < CH; ++c) tma_load_3d(v_smem + vs * DQ_KV_BYTES + c * (DQ_BN * 128), &map_v, &v_full[vs], kvh * p.v_col0_stride + c * 64, row, b);
             }
         }
     } else if (warp == 1 || warp == W_DP) {
@@ -561,7 +565,8 @@ attn_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         const int i = i0 + r;
         const uint32_t lane_addr = tmem_base + ((uint32_t)(q4 * 32) << 16);
         const float sl2 = p.scale * LOG2E;
-        const long long sidx = ((long long)b * p.n_heads + h) * p.seq + i;
+        const int ic = min(i, p.seq - 1);              // rows past the end: a valid row's numbers, nothing of theirs is stored
+        const long long sidx = ((long long)b * p.n_heads + h) * p.seq + ic;
         const float neg_lse2 = -p.lse[sidx] * LOG2E;
         float dlt;
         if (HD == 256 && p.o != nullptr) {
@@ -570,8 +575,8 @@ attn_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             // dK/dV kernel
             {
                 const int part = g0 * 2 + half;
-                const __nv_bfloat16* orow = p.o + (long long)b * p.so_b + (long long)i * p.so_s + (long long)h * p.so_h + part * 64;
-                const __nv_bfloat16* drow = p.d_o + (long long)b * p.sdo_b + (long long)i * p.sdo_s + (long long)h * p.sdo_h + part * 64;
+                const __nv_bfloat16* orow = p.o + (long long)b * p.so_b + (long long)ic * p.so_s + (long long)h * p.so_h + part * 64;
+                const __nv_bfloat16* drow = p.d_o + (long long)b * p.sdo_b + (long long)ic * p.sdo_s + (long long)h * p.sdo_h + part * 64;
                 float a8[8][8], c8[8][8];
 #pragma unroll
                 for (int d = 0; d < 8; ++d) { load8(orow + d * 8, a8[d]); load8(drow + d * 8, c8[d]); }
@@ -584,7 +589,7 @@ attn_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             }
             asm volatile("bar.sync 1, 512;" ::: "memory");     // the 16 element-wise warps
             const float dsum = (delta_smem[r] + delta_smem[BM + r]) + (delta_smem[2 * BM + r] + delta_smem[3 * BM + r]);
-            if (g0 == 0 && half == 0) p.delta_out[sidx] = dsum;
+            if (g0 == 0 && half == 0 && i < p.seq) p.delta_out[sidx] = dsum;
             dlt = dsum;
         } else {
             dlt = p.delta[sidx];
@@ -636,7 +641,7 @@ attn_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                     float t8[8];
 #pragma unroll
                     for (int e = 0; e < 8; ++e) t8[e] = __uint_as_float(o[x + e]) * p.scale;
-                    store8(row + c + x, t8);
+                    if (i < p.seq) store8(row + c + x, t8);
                 }
             }
         }
@@ -692,7 +697,11 @@ __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gmem, u
                  : "memory");
 }
 
-template <int HD>
+// STATS_BULK: the statistics (lse, delta) of a tile's 32 queries come by bulk copy, for which every tile has to start on
+// 128 bytes and end inside its row: sequences that are a multiple of KV_BQ.  Otherwise the TMA warp loads them, one query per
+// lane, before it waits for the stage; queries past the end get lse = inf, so that their probabilities and dS are zero.  (A
+// flag at run time in place of the template cost the bulk form 1 % of the pass at 8 x 4096 tokens, head size 64.)
+template <int HD, bool STATS_BULK>
 __global__ void __launch_bounds__(KvDim<HD>::THREADS, KvDim<HD>::GROUPS == 1 ? 2 : 1)
 attn_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
                    const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const BwdParams p) {
@@ -751,19 +760,43 @@ attn_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     dep_wait();     // set-up above overlapped the previous kernel's tail; its results are needed from here on
 
     if (warp == 0) {
-        if (lane == 0) {
+        const long long srow = ((long long)b * p.n_heads + h) * p.seq;
+        if constexpr (!STATS_BULK) {
+            int st = 0;
+            uint32_t sph = 0;
+            for (int t = 0; t < n_tiles; ++t) {
+                const int i0 = (qs_lo + t) * KV_BQ, i = i0 + lane;
+                const float lse_t = i < p.seq ? p.lse[srow + i] : INFINITY;
+                const float delta_t = i < p.seq ? p.delta[srow + i] : 0.f;
+                if (!warp_wait(&qdo_empty[st], sph ^ 1, abort_flag)) break;
+                stats[st * 2 * KV_BQ + lane] = lse_t;
+                stats[st * 2 * KV_BQ + KV_BQ + lane] = delta_t;
+                __syncwarp();
+                if (lane == 0) {
+                    if (t == 0) {
+                        mbar_arrive_expect_tx(kv_full, 2 * Q_BYTES);
+                        for (int c = 0; c < CH; ++c) tma_load_3d(k_smem + c * (BM * 128), &map_k, kv_full, kvh * p.k_col0_stride + c * 64, j0, b);
+                        for (int c = 0; c < CH; ++c) tma_load_3d(v_smem + c * (BM * 128), &map_v, kv_full, kvh * p.v_col0_stride + c * 64, j0, b);
+                    }
+                    mbar_arrive_expect_tx(&qdo_full[st], 2 * KV_Q_BYTES);
+                    for (int c = 0; c < CH; ++c) tma_load_3d(q_smem + st * KV_Q_BYTES + c * (KV_BQ * 128), &map_q, &qdo_full[st], h * p.q_col0_stride + c * 64, i0, b);
+                    for (int c = 0; c < CH; ++c) tma_load_3d(do_smem + st * KV_Q_BYTES + c * (KV_BQ * 128), &map_do, &qdo_full[st], h * p.do_col0_stride + c * 64, i0, b);
+                }
+                __syncwarp();
+                if (++st == KV_STAGES) { st = 0; sph ^= 1; }
+            }
+        } else if (lane == 0) {
             mbar_arrive_expect_tx(kv_full, 2 * Q_BYTES);
-            for (int c = 0; c < CH; ++c) tma_load_2d(k_smem + c * (BM * 128), &map_k, kv_full, kvh * p.k_col0_stride + c * 64, b * p.seq + j0);
-            for (int c = 0; c < CH; ++c) tma_load_2d(v_smem + c * (BM * 128), &map_v, kv_full, kvh * p.v_col0_stride + c * 64, b * p.seq + j0);
-            const long long srow = ((long long)b * p.n_heads + h) * p.seq;
+            for (int c = 0; c < CH; ++c) tma_load_3d(k_smem + c * (BM * 128), &map_k, kv_full, kvh * p.k_col0_stride + c * 64, j0, b);
+            for (int c = 0; c < CH; ++c) tma_load_3d(v_smem + c * (BM * 128), &map_v, kv_full, kvh * p.v_col0_stride + c * 64, j0, b);
             int st = 0;
             uint32_t sph = 0;                           // stage of tile t and its phase parity (t / KV_STAGES) & 1
             for (int t = 0; t < n_tiles; ++t) {
                 const int i0 = (qs_lo + t) * KV_BQ;
                 if (!mbar_wait(&qdo_empty[st], sph ^ 1, abort_flag)) break;
                 mbar_arrive_expect_tx(&qdo_full[st], 2 * KV_Q_BYTES + KV_STATS_BYTES);
-                for (int c = 0; c < CH; ++c) tma_load_2d(q_smem + st * KV_Q_BYTES + c * (KV_BQ * 128), &map_q, &qdo_full[st], h * p.q_col0_stride + c * 64, b * p.seq + i0);
-                for (int c = 0; c < CH; ++c) tma_load_2d(do_smem + st * KV_Q_BYTES + c * (KV_BQ * 128), &map_do, &qdo_full[st], h * p.do_col0_stride + c * 64, b * p.seq + i0);
+                for (int c = 0; c < CH; ++c) tma_load_3d(q_smem + st * KV_Q_BYTES + c * (KV_BQ * 128), &map_q, &qdo_full[st], h * p.q_col0_stride + c * 64, i0, b);
+                for (int c = 0; c < CH; ++c) tma_load_3d(do_smem + st * KV_Q_BYTES + c * (KV_BQ * 128), &map_do, &qdo_full[st], h * p.do_col0_stride + c * 64, i0, b);
                 bulk_load_1d(stats + st * 2 * KV_BQ, p.lse + srow + i0, KV_BQ * 4, &qdo_full[st]);
                 bulk_load_1d(stats + st * 2 * KV_BQ + KV_BQ, p.delta + srow + i0, KV_BQ * 4, &qdo_full[st]);
                 if (++st == KV_STAGES) { st = 0; sph ^= 1; }
@@ -855,7 +888,11 @@ attn_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             tmem_ld_wait();
             tc_fence_before();
             if (!INPLACE) mbar_arrive(&sdp_free[g]);
-            // lse / delta of the 16 queries (the stage's loads completed before S^T was issued)
+            // lse / delta of the 16 queries (the stage's loads completed before S^T was issued).  Where a warp wrote them,
+            // this wait, which returns at once, orders the reads after its writes
+            if constexpr (!STATS_BULK) {
+                if (!mbar_wait(&qdo_full[t % KV_STAGES], (uint32_t)((t / KV_STAGES) & 1), abort_flag)) { ok = false; break; }
+            }
             const float* st_l = stats + (t % KV_STAGES) * 2 * KV_BQ + half * 16;
             const float* st_d = st_l + KV_BQ;
             const bool need_mask = (i0 < j0 + BM - 1) || (p.window > 0 && i0 + 15 - j0 >= p.window);
@@ -901,13 +938,13 @@ attn_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 tmem_ld_32x32(lane_addr + KV_DK_COL + half * (ACC / 2) + c, o);
                 tmem_ld_wait();
 #pragma unroll
-                for (int x = 0; x < 32; x += 4)
+                for (int x = 0; x < 32 && j < p.seq; x += 4)
                     atomicAdd(reinterpret_cast<float4*>(krow + c + x), make_float4(__uint_as_float(o[x]) * p.scale, __uint_as_float(o[x + 1]) * p.scale,
                                                                                  __uint_as_float(o[x + 2]) * p.scale, __uint_as_float(o[x + 3]) * p.scale));
                 tmem_ld_32x32(lane_addr + KV_DV_COL + half * (ACC / 2) + c, o);
                 tmem_ld_wait();
 #pragma unroll
-                for (int x = 0; x < 32; x += 4)
+                for (int x = 0; x < 32 && j < p.seq; x += 4)
                     atomicAdd(reinterpret_cast<float4*>(vrow + c + x), make_float4(__uint_as_float(o[x]), __uint_as_float(o[x + 1]),
                                                                                  __uint_as_float(o[x + 2]), __uint_as_float(o[x + 3])));
             }
@@ -950,63 +987,78 @@ int32_t launch_dq(const CUtensorMap& mq, const CUtensorMap& md, const CUtensorMa
     MFT_LAUNCH_CHECK("attn_dq_tc");
     return MFT_OK;
 }
-template <int HD>
-int32_t launch_dkv(const CUtensorMap& mq, const CUtensorMap& md, const CUtensorMap& mk, const CUtensorMap& mv, const BwdParams& p, int seq, int n_heads, int batch,
+template <int HD, bool STATS_BULK>
+int32_t launch_dkv_as(const CUtensorMap& mq, const CUtensorMap& md, const CUtensorMap& mk, const CUtensorMap& mv, const BwdParams& p, int seq, int n_heads, int batch,
                    cudaStream_t stream) {
     static PerDeviceFlag configured_on;           // function attributes are per device
     bool& configured = configured_on.here();
     if (!configured) {
-        if (int32_t s = check_cuda(cudaFuncSetAttribute(attn_dkv_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, KvDim<HD>::SMEM), "attention smem attribute")) return s;
+        if (int32_t s = check_cuda(cudaFuncSetAttribute(attn_dkv_tc_kernel<HD, STATS_BULK>, cudaFuncAttributeMaxDynamicSharedMemorySize, KvDim<HD>::SMEM), "attention smem attribute")) return s;
         configured = true;
     }
-    dim3 grid((unsigned)(seq / BM), (unsigned)(KvDim<HD>::NPART * n_heads), (unsigned)batch);
-    launch_dep(attn_dkv_tc_kernel<HD>, dim3(grid), dim3(KvDim<HD>::THREADS), (size_t)(KvDim<HD>::SMEM), stream, mq, md, mk, mv, p);
+    dim3 grid((unsigned)((seq + BM - 1) / BM), (unsigned)(KvDim<HD>::NPART * n_heads), (unsigned)batch);
+    launch_dep(attn_dkv_tc_kernel<HD, STATS_BULK>, dim3(grid), dim3(KvDim<HD>::THREADS), (size_t)(KvDim<HD>::SMEM), stream, mq, md, mk, mv, p);
     MFT_LAUNCH_CHECK("attn_dkv_tc");
     return MFT_OK;
 }
+template <int HD>
+int32_t launch_dkv(const CUtensorMap& mq, const CUtensorMap& md, const CUtensorMap& mk, const CUtensorMap& mv, const BwdParams& p, int seq, int n_heads, int batch,
+                   cudaStream_t stream) {
+    return seq % KV_BQ == 0 ? launch_dkv_as<HD, true>(mq, md, mk, mv, p, seq, n_heads, batch, stream)
+                            : launch_dkv_as<HD, false>(mq, md, mk, mv, p, seq, n_heads, batch, stream);
+}
+
+// Where the backward kernels win over the mma.sync pair.  Microseconds mma.sync / tcgen05 of the whole backward pass, batch
+// 4 and 8:  head size 256, 4 heads:   64 tokens 28.6 / 25.5, 29.4 / 26.1;  128: 40.1 / 37.9, 41.6 / 40.2;  1000: 275 / 126, 433 / 211
+//   128, 8 heads:   128 tokens 29.4 / 30.5, 31.3 / 32.1;  160: 36.7 / 30.8, 48.1 / 33.7;  1000: 277 / 127, 476 / 211
+//   64, 14 / 2 heads:   160 tokens 33.2 / 31.4, 41.9 / 41.9;  200: 39.6 / 33.1, 54.2 / 44.0;  1000: 236 / 136, 403 / 224
+//   64, 12 / 12 heads:  160 tokens 25.8 / 26.0, 32.0 / 34.8;  200: 34.9 / 33.1, 44.8 / 45.0;  1000: 203 / 178, 345 / 295
+bool bwd_long_enough(int hd, int seq) { return hd == 256 || seq > (hd == 128 ? 128 : 192); }
 #define HD_DISPATCH(hd, CALL64, CALL128, CALL256) ((hd) == 64 ? (CALL64) : (hd) == 128 ? (CALL128) : (CALL256))
 
 }  // namespace
 
 int32_t attn_fwd_sm100(const AttnParams& a, int hd, cudaStream_t stream) {
     static const int enabled = [] { const char* e = std::getenv("MFT_ATTN_TC"); return e ? std::atoi(e) : 1; }();
-    if (!enabled || !tc_shape_ok(hd) || a.seq % BM != 0 || !device_status_word()) return MFT_ERR_UNSUPPORTED;
-    // measured (batch 8, 14 / 2 heads of 64): at 256 tokens the mma.sync forward is faster (0.0205 against 0.0225 ms),
-    // from 512 tokens on this kernel wins (0.039 against 0.041 ms, 2.3 x at 4096); MFT_ATTN_TC=2 forces it
-    if (hd != 256 && a.seq < 512 && enabled < 2) return MFT_ERR_UNSUPPORTED;
+    if (!enabled || !tc_shape_ok(hd) || !device_status_word()) return MFT_ERR_UNSUPPORTED;
+    if (!(a.scale > 0.f)) return MFT_ERR_UNSUPPORTED;      // the running maximum is taken before the scaling
+    // A 128-query tile of this kernel against two 64-query CTAs of the mma.sync one: short sequences are bound by the
+    // latency of one tile's chain (tens of barriers), where the smaller CTAs win.  Crossing points, microseconds mma.sync /
+    // tcgen05 (batch 4 and 8):  head size 256, 4 heads:   256 tokens 17.9 / 18.0, 18.0 / 18.1;  300: 20.5 / 18.1, 25.9 / 18.4
+    //   128, 8 heads:   128 tokens 8.0 / 9.6, 8.1 / 10.0;  160: 9.7 / 9.7, 12.8 / 10.0
+    //   64, 14 heads:   384 tokens 18.2 / 17.1, 24.0 / 25.6;  437: 19.6 / 18.2, 30.6 / 29.8
+    // and 113 / 49, 110 / 57, 100 / 66 at 8 x 1000.  MFT_ATTN_TC=2 forces it.
+    if (a.seq <= (hd == 256 ? 256 : hd == 128 ? 128 : 384) && enabled < 2) return MFT_ERR_UNSUPPORTED;
     if (!token_major(a.sq, a.seq) || !token_major(a.sk, a.seq) || !token_major(a.sv, a.seq)) return MFT_ERR_UNSUPPORTED;
     if (a.sq.stride_h % 8 || a.sk.stride_h % 8 || a.sv.stride_h % 8 || a.so.stride_s % 8 || a.so.stride_h % 8 || a.so.stride_b % 8) return MFT_ERR_UNSUPPORTED;
     if ((int64_t)a.batch * a.seq >= (1ll << 31)) return MFT_ERR_UNSUPPORTED;
     CUtensorMap mq, mk, mv;
-    const int64_t rows = (int64_t)a.batch * a.seq;
-    if (make_tmap_bf16(&mq, a.q, rows, (int64_t)(a.n_heads - 1) * a.sq.stride_h + hd, a.sq.stride_s, BM) != MFT_OK) return MFT_ERR_UNSUPPORTED;
-    if (make_tmap_bf16(&mk, a.k, rows, (int64_t)(a.n_kv - 1) * a.sk.stride_h + hd, a.sk.stride_s, BN) != MFT_OK) return MFT_ERR_UNSUPPORTED;
-    if (make_tmap_bf16(&mv, a.v, rows, (int64_t)(a.n_kv - 1) * a.sv.stride_h + hd, a.sv.stride_s, BN) != MFT_OK) return MFT_ERR_UNSUPPORTED;
+    if (make_tmap_bf16_batched(&mq, a.q, a.batch, a.seq, (int64_t)(a.n_heads - 1) * a.sq.stride_h + hd, a.sq.stride_s, BM) != MFT_OK) return MFT_ERR_UNSUPPORTED;
+    if (make_tmap_bf16_batched(&mk, a.k, a.batch, a.seq, (int64_t)(a.n_kv - 1) * a.sk.stride_h + hd, a.sk.stride_s, BN) != MFT_OK) return MFT_ERR_UNSUPPORTED;
+    if (make_tmap_bf16_batched(&mv, a.v, a.batch, a.seq, (int64_t)(a.n_kv - 1) * a.sv.stride_h + hd, a.sv.stride_s, BN) != MFT_OK) return MFT_ERR_UNSUPPORTED;
     if (a.sk.stride_h != a.sv.stride_h) return MFT_ERR_UNSUPPORTED;
     FwdParams p{};
     p.seq = a.seq; p.n_heads = a.n_heads; p.rep = a.rep; p.window = a.window; p.scale = a.scale;
     p.out = a.out; p.so_b = a.so.stride_b; p.so_s = a.so.stride_s; p.so_h = a.so.stride_h; p.lse = a.lse;
     p.status = device_status_word();
     p.q_col0_stride = (int)a.sq.stride_h; p.kv_col0_stride = (int)a.sk.stride_h;
-    dim3 grid((unsigned)(a.seq / BM), (unsigned)a.n_heads, (unsigned)a.batch);
+    dim3 grid((unsigned)((a.seq + BM - 1) / BM), (unsigned)a.n_heads, (unsigned)a.batch);
     return HD_DISPATCH(hd, launch_fwd<64>(mq, mk, mv, p, grid, stream), launch_fwd<128>(mq, mk, mv, p, grid, stream), launch_fwd<256>(mq, mk, mv, p, grid, stream));
 }
 
 int32_t attn_dq_sm100(const AttnParams& a, int hd, bool compute_delta, cudaStream_t stream) {
     static const int enabled = [] { const char* e = std::getenv("MFT_ATTN_TC"); return e ? std::atoi(e) : 1; }();
-    if (!enabled || !tc_shape_ok(hd) || a.seq % BM != 0 || !device_status_word()) return MFT_ERR_UNSUPPORTED;
-    // the backward kernels win from 256 tokens on (0.064 against 0.073 ms at 256, 2.6 x at 4096); MFT_ATTN_TC=2 forces them
-    if (hd != 256 && a.seq < 256 && enabled < 2) return MFT_ERR_UNSUPPORTED;
+    if (!enabled || !tc_shape_ok(hd) || !device_status_word()) return MFT_ERR_UNSUPPORTED;
+    if (!bwd_long_enough(hd, a.seq) && enabled < 2) return MFT_ERR_UNSUPPORTED;
     if (compute_delta && hd != 256) return MFT_ERR_UNSUPPORTED;
     if (!token_major(a.sq, a.seq) || !token_major(a.sk, a.seq) || !token_major(a.sv, a.seq) || !token_major(a.sdo, a.seq)) return MFT_ERR_UNSUPPORTED;
     if (a.sq.stride_h % 8 || a.sk.stride_h % 8 || a.sv.stride_h % 8 || a.sdo.stride_h % 8) return MFT_ERR_UNSUPPORTED;
     if ((int64_t)a.batch * a.seq >= (1ll << 31)) return MFT_ERR_UNSUPPORTED;
     CUtensorMap mq, md, mk, mv;
-    const int64_t rows = (int64_t)a.batch * a.seq;
-    if (make_tmap_bf16(&mq, a.q, rows, (int64_t)(a.n_heads - 1) * a.sq.stride_h + hd, a.sq.stride_s, BM) != MFT_OK) return MFT_ERR_UNSUPPORTED;
-    if (make_tmap_bf16(&md, a.d_o, rows, (int64_t)(a.n_heads - 1) * a.sdo.stride_h + hd, a.sdo.stride_s, BM) != MFT_OK) return MFT_ERR_UNSUPPORTED;
-    if (make_tmap_bf16(&mk, a.k, rows, (int64_t)(a.n_kv - 1) * a.sk.stride_h + hd, a.sk.stride_s, DQ_BN) != MFT_OK) return MFT_ERR_UNSUPPORTED;
-    if (make_tmap_bf16(&mv, a.v, rows, (int64_t)(a.n_kv - 1) * a.sv.stride_h + hd, a.sv.stride_s, DQ_BN) != MFT_OK) return MFT_ERR_UNSUPPORTED;
+    if (make_tmap_bf16_batched(&mq, a.q, a.batch, a.seq, (int64_t)(a.n_heads - 1) * a.sq.stride_h + hd, a.sq.stride_s, BM) != MFT_OK) return MFT_ERR_UNSUPPORTED;
+    if (make_tmap_bf16_batched(&md, a.d_o, a.batch, a.seq, (int64_t)(a.n_heads - 1) * a.sdo.stride_h + hd, a.sdo.stride_s, BM) != MFT_OK) return MFT_ERR_UNSUPPORTED;
+    if (make_tmap_bf16_batched(&mk, a.k, a.batch, a.seq, (int64_t)(a.n_kv - 1) * a.sk.stride_h + hd, a.sk.stride_s, DQ_BN) != MFT_OK) return MFT_ERR_UNSUPPORTED;
+    if (make_tmap_bf16_batched(&mv, a.v, a.batch, a.seq, (int64_t)(a.n_kv - 1) * a.sv.stride_h + hd, a.sv.stride_s, DQ_BN) != MFT_OK) return MFT_ERR_UNSUPPORTED;
     BwdParams p{};
     p.seq = a.seq; p.n_heads = a.n_heads; p.n_kv = a.n_kv; p.rep = a.rep; p.window = a.window; p.scale = a.scale;
     p.lse = a.lse; p.delta = a.delta; p.dq = a.dq; p.sq_b = a.sq.stride_b; p.sq_s = a.sq.stride_s; p.sq_h = a.sq.stride_h;
@@ -1019,25 +1071,23 @@ int32_t attn_dq_sm100(const AttnParams& a, int hd, bool compute_delta, cudaStrea
         p.so_b = a.so.stride_b; p.so_s = a.so.stride_s; p.so_h = a.so.stride_h;
         p.sdo_b = a.sdo.stride_b; p.sdo_s = a.sdo.stride_s; p.sdo_h = a.sdo.stride_h;
     }
-    dim3 grid((unsigned)(a.seq / BM), (unsigned)a.n_heads, (unsigned)a.batch);
+    dim3 grid((unsigned)((a.seq + BM - 1) / BM), (unsigned)a.n_heads, (unsigned)a.batch);
     return HD_DISPATCH(hd, launch_dq<64>(mq, md, mk, mv, p, grid, stream), launch_dq<128>(mq, md, mk, mv, p, grid, stream), launch_dq<256>(mq, md, mk, mv, p, grid, stream));
 }
 
 int32_t attn_dkv_sm100(const AttnParams& a, int hd, cudaStream_t stream) {
     static const int enabled = [] { const char* e = std::getenv("MFT_ATTN_TC"); return e ? std::atoi(e) : 1; }();
-    if (!enabled || !tc_shape_ok(hd) || a.seq % BM != 0 || !a.dkv_acc || !device_status_word()) return MFT_ERR_UNSUPPORTED;
-    // the backward kernels win from 256 tokens on (0.064 against 0.073 ms at 256, 2.6 x at 4096); MFT_ATTN_TC=2 forces them
-    if (hd != 256 && a.seq < 256 && enabled < 2) return MFT_ERR_UNSUPPORTED;
+    if (!enabled || !tc_shape_ok(hd) || !a.dkv_acc || !device_status_word()) return MFT_ERR_UNSUPPORTED;
+    if (!bwd_long_enough(hd, a.seq) && enabled < 2) return MFT_ERR_UNSUPPORTED;
     if (!token_major(a.sq, a.seq) || !token_major(a.sk, a.seq) || !token_major(a.sv, a.seq) || !token_major(a.sdo, a.seq)) return MFT_ERR_UNSUPPORTED;
     if (a.sq.stride_h % 8 || a.sk.stride_h % 8 || a.sv.stride_h % 8 || a.sdo.stride_h % 8) return MFT_ERR_UNSUPPORTED;
     if ((int64_t)a.batch * a.seq >= (1ll << 31) || 2 * a.n_heads > 65535) return MFT_ERR_UNSUPPORTED;
     if (reinterpret_cast<uintptr_t>(a.lse) % 16 || reinterpret_cast<uintptr_t>(a.delta) % 16 || reinterpret_cast<uintptr_t>(a.dkv_acc) % 16) return MFT_ERR_UNSUPPORTED;
     CUtensorMap mq, md, mk, mv;
-    const int64_t rows = (int64_t)a.batch * a.seq;
-    if (make_tmap_bf16(&mq, a.q, rows, (int64_t)(a.n_heads - 1) * a.sq.stride_h + hd, a.sq.stride_s, KV_BQ) != MFT_OK) return MFT_ERR_UNSUPPORTED;
-    if (make_tmap_bf16(&md, a.d_o, rows, (int64_t)(a.n_heads - 1) * a.sdo.stride_h + hd, a.sdo.stride_s, KV_BQ) != MFT_OK) return MFT_ERR_UNSUPPORTED;
-    if (make_tmap_bf16(&mk, a.k, rows, (int64_t)(a.n_kv - 1) * a.sk.stride_h + hd, a.sk.stride_s, BM) != MFT_OK) return MFT_ERR_UNSUPPORTED;
-    if (make_tmap_bf16(&mv, a.v, rows, (int64_t)(a.n_kv - 1) * a.sv.stride_h + hd, a.sv.stride_s, BM) != MFT_OK) return MFT_ERR_UNSUPPORTED;
+    if (make_tmap_bf16_batched(&mq, a.q, a.batch, a.seq, (int64_t)(a.n_heads - 1) * a.sq.stride_h + hd, a.sq.stride_s, KV_BQ) != MFT_OK) return MFT_ERR_UNSUPPORTED;
+    if (make_tmap_bf16_batched(&md, a.d_o, a.batch, a.seq, (int64_t)(a.n_heads - 1) * a.sdo.stride_h + hd, a.sdo.stride_s, KV_BQ) != MFT_OK) return MFT_ERR_UNSUPPORTED;
+    if (make_tmap_bf16_batched(&mk, a.k, a.batch, a.seq, (int64_t)(a.n_kv - 1) * a.sk.stride_h + hd, a.sk.stride_s, BM) != MFT_OK) return MFT_ERR_UNSUPPORTED;
+    if (make_tmap_bf16_batched(&mv, a.v, a.batch, a.seq, (int64_t)(a.n_kv - 1) * a.sv.stride_h + hd, a.sv.stride_s, BM) != MFT_OK) return MFT_ERR_UNSUPPORTED;
     BwdParams p{};
     p.seq = a.seq; p.n_heads = a.n_heads; p.n_kv = a.n_kv; p.rep = a.rep; p.window = a.window; p.scale = a.scale;
     p.lse = a.lse; p.delta = a.delta; p.dq = a.dq; p.sq_b = a.sq.stride_b; p.sq_s = a.sq.stride_s; p.sq_h = a.sq.stride_h;

@@ -358,24 +358,32 @@ static TmapSlot* tmap_slot(const TmapKey& k) {
     return &table[(size_t)((h >> 40) % TMAP_SLOTS)];
 }
 
-int32_t make_tmap_bf16(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_rows) {
-    const TmapKey key{base, rows, cols, ld, box_rows, 0};
+static int32_t make_tmap_bf16_3d(CUtensorMap* map, const void* base, int64_t batch, int64_t rows, int64_t cols, int64_t ld, int box_rows, bool batched) {
+    const TmapKey key{base, rows, cols, ld, box_rows, batched ? (int32_t)(1 + batch) : 0};
     TmapSlot* slot = tmap_slot(key);
     if (slot->used && slot->key == key) { *map = slot->map; return MFT_OK; }
     EncodeTiledFn enc = get_encode();
     if (!enc) return fail(MFT_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
     if (reinterpret_cast<uintptr_t>(base) % 16 != 0) return fail(MFT_ERR_INVALID_ARG, "GEMM operand base must be 16-byte aligned");
     if (ld % 8 != 0) return fail(MFT_ERR_INVALID_ARG, "GEMM operand row stride must be a multiple of 8 elements");
-    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    cuuint32_t box[2] = {(cuuint32_t)GEMM_BK, (cuuint32_t)box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+    cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)batch};
+    cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)rows * (cuuint64_t)ld * 2};
+    cuuint32_t box[3] = {(cuuint32_t)GEMM_BK, (cuuint32_t)box_rows, 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, batched ? 3 : 2, const_cast<void*>(base), dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(MFT_ERR_CUDA, "cuTensorMapEncodeTiled failed with code " + std::to_string((int)r));
     slot->key = key; slot->map = *map; slot->used = true;
     return MFT_OK;
+}
+
+int32_t make_tmap_bf16(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_rows) {
+    return make_tmap_bf16_3d(map, base, 1, rows, cols, ld, box_rows, false);
+}
+
+int32_t make_tmap_bf16_batched(CUtensorMap* map, const void* base, int64_t batch, int64_t rows, int64_t cols, int64_t ld, int box_rows) {
+    return make_tmap_bf16_3d(map, base, batch, rows, cols, ld, box_rows, true);
 }
 
 // Tensor map over a row-major f32 matrix [rows, cols]: box = {32 columns, 32 rows}, 128-byte swizzle.

@@ -101,6 +101,8 @@ int32_t gemm_nt_run_ksplit(const GemmCall& c, cudaStream_t stream);
 // multiple of 384), or 0 when the pair kernel does not take the call
 int gemm_nt_pair_tile_cols(int64_t m, int64_t n, int64_t k, int64_t k2, bool d_is_f32);
 int32_t make_tmap_bf16(struct CUtensorMap_st* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_rows);
+// [batch, rows, cols] with the batches rows * ld elements apart; a box lies in one batch, rows past its end read as zeros
+int32_t make_tmap_bf16_batched(struct CUtensorMap_st* map, const void* base, int64_t batch, int64_t rows, int64_t cols, int64_t ld, int box_rows);
 int32_t make_tmap_f32_out(struct CUtensorMap_st* map, const void* base, int64_t rows, int64_t cols, int64_t ld);
 int num_sms();
 bool gemm_profiling_enabled();       // per-launch event timing is on (incompatible with stream capture)

@@ -1,0 +1,49 @@
+"""tcgen05 attention kernels on sequences that are no multiple of their 128-row tiles, against f32 torch."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _reference(q, k, v, d_o, scale, window):
+    q, k, v = (x.float().detach().requires_grad_() for x in (q, k, v))
+    rep, s = q.shape[1] // k.shape[1], q.shape[2]
+    kk, vv = k.repeat_interleave(rep, 1), v.repeat_interleave(rep, 1)
+    i, j = torch.arange(s, device=q.device)[:, None], torch.arange(s, device=q.device)[None, :]
+    mask = (j <= i) & ((i - j < window) if window > 0 else True)
+    logits = (q @ kk.transpose(-1, -2) * scale).masked_fill(~mask, float("-inf"))
+    o = logits.softmax(-1) @ vv
+    grads = torch.autograd.grad(o, (q, k, v), d_o.float())
+    return (o, logits.logsumexp(-1), *grads)
+
+
+# around the 128-row tile, the 64- / 32-key and 32-query tiles, the 32-query rule of the statistics' bulk copy, and both
+# sides of the lengths from which the kernels are taken
+@pytest.mark.parametrize("hd,heads,kv,seq,window", [
+    (256, 4, 1, 2, 0), (256, 4, 1, 31, 0), (256, 4, 1, 97, 33), (256, 2, 1, 127, 0), (256, 4, 1, 129, 0), (256, 4, 1, 161, 64),
+    (256, 4, 1, 256, 0), (256, 4, 1, 257, 0), (256, 4, 1, 1001, 512), (256, 4, 2, 640 + 32, 100), (64, 14, 2, 193, 0), (64, 14, 2, 385, 0),
+    (64, 4, 2, 513, 0), (64, 4, 2, 544, 0), (64, 4, 1, 1023, 70), (128, 4, 2, 129, 0), (128, 4, 2, 600, 0), (128, 2, 1, 515, 96)])
+def test_ragged_sequences(hd, heads, kv, seq, window):
+    from mobilefinetuner_b200 import ops as O
+    g = torch.Generator(device="cuda").manual_seed(seq)
+
+    def rnd(n):
+        return torch.randn(3, seq, n, hd, device="cuda", generator=g).bfloat16().permute(0, 2, 1, 3)
+    q, k, v, d_o = rnd(heads), rnd(kv), rnd(kv), rnd(heads)
+    # the sample in the middle is not a number: none of it may reach its neighbours through a tile's rows past the end
+    for x in (q, k, v, d_o):
+        x[1] = float("nan")
+    scale = hd ** -0.5
+    o, lse = O.attention_fwd(q, k, v, scale, window)
+    got = (o, lse, *O.attention_bwd(q, k, v, o, d_o, lse, scale, window))
+    keep = [0, 2]
+    ref = _reference(q[keep], k[keep], v[keep], d_o[keep], scale, window)
+    for name, a, b in zip(("o", "lse", "dq", "dk", "dv"), got, ref):
+        a = a[keep].float()
+        assert torch.isfinite(a).all(), name
+        # P, dS and the results are rounded to bf16 (2^-9 each, sums of independent roundings below): 4 * 2^-9
+        assert (a - b).norm() <= 2 ** -7 * b.norm(), (name, ((a - b).norm() / b.norm()).item())
+        # no row is off on its own (rows of a few keys carry the full rounding of their terms)
+        row = (a - b).norm(dim=-1) if a.dim() == 4 else (a - b).abs()
+        size = b.norm(dim=-1) if a.dim() == 4 else b.abs()
+        assert (row <= 2 ** -5 * (size + size.mean())).all(), name
