@@ -123,285 +123,213 @@ rmsnorm_bwd_kernel(const TDY* __restrict__ dy, const TX* __restrict__ x, const f
 }
 
 
-// ---------------------------------------------------------------- RMSNorm, one warp per row (dim <= 256 * VPL)
-constexpr int NORM_WARPS = 8;     // rows per CTA
+// ---------------------------------------------------------------- RMSNorm, a CTA (or a few of its warps) per row, eight columns per thread (dim <= 2048)
+// Bound by HBM on long inputs and by one chain of load -> row sum -> load -> row sum on short ones.  A thread holds one
+// 8-vector of every input of its row, so that all loads of the row are in flight before the first sum; a row of 640 / 896 /
+// 1152 columns takes 3 / 4 / 5 warps and an SM keeps a dozen rows going.  (One warp per row with five vectors a lane left
+// most SMs idle below a few thousand rows and could not hold every input, so the second half of the loads waited for a sum.)
+constexpr int ROW_MAX_DIM = 2048, ROW_MAX_WARPS = ROW_MAX_DIM / 256;
+constexpr int ROW_SLOTS = ROW_MAX_WARPS;          // warps of a CTA: one row of up to eight, or up to four rows of one or two
 
-template <typename TX, typename TY, int VPL>
-__global__ void __launch_bounds__(NORM_WARPS * 32)
-rmsnorm_fwd_warp_kernel(const TX* __restrict__ x, const float* __restrict__ w, float eps, int unit_offset,
-                        TY* __restrict__ y, float* __restrict__ rstd_out, const float* __restrict__ residual,
-                        float* __restrict__ sum_out, int64_t rows, int64_t dim) {
+// rows of up to 256 / 512 columns share a CTA of four warps
+inline dim3 row_block(int64_t dim) {
+    const unsigned x = (unsigned)((dim / 8 + 31) / 32 * 32);
+    return dim3(x, x <= 64 ? 128 / x : 1);
+}
+inline dim3 row_grid(int64_t rows, int64_t dim) { const int64_t y = row_block(dim).y; return dim3((unsigned)((rows + y - 1) / y)); }
+
+// sum over a row's threads; `slots` is used once per kernel, so no barrier is needed behind the reads
+__device__ __forceinline__ float row_sum(float v, float* slots) {
+    v = warp_sum(v);
+    const int warps = blockDim.x >> 5;
+    slots += threadIdx.y * warps;
+    if ((threadIdx.x & 31) == 0) slots[threadIdx.x >> 5] = v;
+    __syncthreads();
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < ROW_MAX_WARPS; ++i) if (i < warps) s += slots[i];
+    return s;
+}
+// The fused kernels below give the same bits as the separate ones: no contraction is left to the compiler.
+__device__ __forceinline__ float norm_out(float v, float rstd, float w) { return __fmul_rn(__fmul_rn(v, rstd), w); }
+__device__ __forceinline__ float norm_grad(float g, float rstd, float x, float coeff) { return __fmaf_rn(g, rstd, -__fmul_rn(x, coeff)); }
+__device__ __forceinline__ void zero8(float (&v)[8]) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = 0.f;
+}
+
+template <typename TX, typename TY>
+__global__ void __launch_bounds__(ROW_MAX_WARPS * 32)
+rmsnorm_fwd_row_kernel(const TX* __restrict__ x, const float* __restrict__ w, float eps, int unit_offset,
+                       TY* __restrict__ y, float* __restrict__ rstd_out, const float* __restrict__ residual,
+                       float* __restrict__ sum_out, int64_t rows, int64_t dim) {
     dep_trigger();
     dep_wait();
-    const int lane = threadIdx.x & 31;
-    const int64_t row = (int64_t)blockIdx.x * NORM_WARPS + (threadIdx.x >> 5);
-    if (row >= rows) return;
-    const TX* xr = x + row * dim;
-    const int nvec = (int)(dim / 8);
-    float v[VPL][8];
-    float ss = 0.f;
-#pragma unroll
-    for (int k = 0; k < VPL; ++k) {
-        const int i = lane + k * 32;
-        if (i < nvec) load8(xr + i * 8, v[k]);
+    __shared__ float s0[ROW_SLOTS];
+    const int i = threadIdx.x * 8;
+    const int64_t row = (int64_t)blockIdx.x * blockDim.y + threadIdx.y, at = row * dim + i;
+    const bool in = row < rows && i < dim;
+    float v[8], wv[8], r[8], ss = 0.f;
+    zero8(v);
+    if (in) {
+        load8(x + at, v);
+        load8(w + i, wv);
+        if (residual) load8(residual + at, r);
     }
 #pragma unroll
-    for (int k = 0; k < VPL; ++k) {
-        if (lane + k * 32 < nvec) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) ss += v[k][j] * v[k][j];
-        }
-    }
-    ss = warp_sum(ss);
+    for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
+    ss = row_sum(ss, s0);
     const float rstd = rsqrtf(ss / (float)dim + eps);
-    if (lane == 0 && rstd_out) rstd_out[row] = rstd;
+    if (threadIdx.x == 0 && in && rstd_out) rstd_out[row] = rstd;
+    if (!in) return;
+    float o[8];
 #pragma unroll
-    for (int k = 0; k < VPL; ++k) {
-        const int i = lane + k * 32;
-        if (i < nvec) {
-            float wv[8], o[8];
-            load8(w + i * 8, wv);
+    for (int j = 0; j < 8; ++j) o[j] = norm_out(v[j], rstd, unit_offset ? 1.0f + wv[j] : wv[j]);
+    if (y) store8(y + at, o);
+    if (residual) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] = v[k][j] * rstd * (unit_offset ? 1.0f + wv[j] : wv[j]);
-            if (y) store8(y + row * dim + i * 8, o);
-            if (residual) {
-                float r[8];
-                load8(residual + row * dim + i * 8, r);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) r[j] += o[j];
-                store8(sum_out + row * dim + i * 8, r);
-            }
-        }
+        for (int j = 0; j < 8; ++j) r[j] = __fadd_rn(r[j], o[j]);
+        store8(sum_out + at, r);
     }
 }
 
-template <typename TDY, typename TX, typename TDX, int VPL>
-__global__ void __launch_bounds__(NORM_WARPS * 32)
-rmsnorm_bwd_warp_kernel(const TDY* __restrict__ dy, const TX* __restrict__ x, const float* __restrict__ w,
-                        const float* __restrict__ rstd_in, float eps, int unit_offset, TDX* __restrict__ dx,
-                        int accumulate, float* __restrict__ dweight, int64_t rows, int64_t dim) {
+template <typename TDY, typename TX, typename TDX>
+__global__ void __launch_bounds__(ROW_MAX_WARPS * 32)
+rmsnorm_bwd_row_kernel(const TDY* __restrict__ dy, const TX* __restrict__ x, const float* __restrict__ w,
+                       const float* __restrict__ rstd_in, float eps, int unit_offset, TDX* __restrict__ dx,
+                       int accumulate, float* __restrict__ dweight, int64_t rows, int64_t dim) {
     dep_trigger();
     dep_wait();
-    const int lane = threadIdx.x & 31;
-    const int64_t row = (int64_t)blockIdx.x * NORM_WARPS + (threadIdx.x >> 5);
-    if (row >= rows) return;
-    const int nvec = (int)(dim / 8);
-    float xv[VPL][8], g[VPL][8];
-#pragma unroll
-    for (int k = 0; k < VPL; ++k) {
-        const int i = lane + k * 32;
-        if (i < nvec) {
-            load8(x + row * dim + i * 8, xv[k]);
-            load8(dy + row * dim + i * 8, g[k]);
-        }
+    __shared__ float s0[ROW_SLOTS], s1[ROW_SLOTS];
+    const int i = threadIdx.x * 8;
+    const int64_t row = (int64_t)blockIdx.x * blockDim.y + threadIdx.y, at = row * dim + i;
+    const bool in = row < rows && i < dim;
+    float xv[8], g[8], wv[8], prev[8];
+    zero8(xv); zero8(g); zero8(wv); zero8(prev);
+    if (in) {
+        load8(x + at, xv);
+        load8(dy + at, g);
+        load8(w + i, wv);
+        if (accumulate) load8(dx + at, prev);
     }
-    const float rs_in = rstd_in ? rstd_in[row] : 0.f;
+    const float rs_in = rstd_in && row < rows ? rstd_in[row] : 0.f;
     float ss = 0.f, dot = 0.f;
 #pragma unroll
-    for (int k = 0; k < VPL; ++k) {
-        const int i = lane + k * 32;
-        if (i < nvec) {
-            float wv[8];
-            load8(w + i * 8, wv);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                if (dweight) atomicAdd(dweight + i * 8 + j, g[k][j] * xv[k][j] * rs_in);
-                g[k][j] *= (unit_offset ? 1.0f + wv[j] : wv[j]);
-                dot += g[k][j] * xv[k][j];
-                ss += xv[k][j] * xv[k][j];
-            }
-        }
+    for (int j = 0; j < 8; ++j) {
+        if (dweight && in) atomicAdd(dweight + i + j, g[j] * xv[j] * rs_in);
+        g[j] *= (unit_offset ? 1.0f + wv[j] : wv[j]);
+        dot += g[j] * xv[j];
+        ss += xv[j] * xv[j];
     }
-    dot = warp_sum(dot);
+    dot = row_sum(dot, s0);
     float rstd = rs_in;
-    if (!rstd_in) rstd = rsqrtf(warp_sum(ss) / (float)dim + eps);
+    if (!rstd_in) rstd = rsqrtf(row_sum(ss, s1) / (float)dim + eps);
     const float coeff = rstd * rstd * rstd / (float)dim * dot;
+    if (!in) return;
+    float o[8];
 #pragma unroll
-    for (int k = 0; k < VPL; ++k) {
-        const int i = lane + k * 32;
-        if (i < nvec) {
-            float o[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] = g[k][j] * rstd - xv[k][j] * coeff;
-            if (accumulate) {
-                float prev[8];
-                load8(dx + row * dim + i * 8, prev);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) o[j] += prev[j];
-            }
-            store8(dx + row * dim + i * 8, o);
-        }
+    for (int j = 0; j < 8; ++j) {
+        o[j] = norm_grad(g[j], rstd, xv[j], coeff);
+        if (accumulate) o[j] = __fadd_rn(o[j], prev[j]);
     }
+    store8(dx + at, o);
 }
-
-
-// Ask for the 32 bytes at p early (no register is held): the fused norm kernels read some rows only after a
-// warp reduction, and without this their latency adds to that of the first loads.
-__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" :: "l"(p)); }
 
 // ---------------------------------------------------------------- fused post-norm + residual add + next pre-norm
 // Gemma wraps every block as  x_sum = x + rms(y_branch) ,  h_next = rms(x_sum)  (post-norm of one block, residual
-// add, pre-norm of the next).  One warp per row keeps x_sum in registers between the two norms, so x_sum is
+// add, pre-norm of the next).  x_sum stays in registers between the two norms, so it is
 // written once and never re-read: same arithmetic, in the same order, as the two separate kernels.
-template <int VPL>
-__global__ void __launch_bounds__(NORM_WARPS * 32)
+__global__ void __launch_bounds__(ROW_MAX_WARPS * 32)
 rmsnorm_add_norm_fwd_kernel(const __nv_bfloat16* __restrict__ y, const float* __restrict__ w_post, int unit_post,
                             const float* __restrict__ residual, const float* __restrict__ w_next, int unit_next, float eps,
                             float* __restrict__ sum_out, float* __restrict__ rstd_post, __nv_bfloat16* __restrict__ h_next,
                             float* __restrict__ rstd_next, int64_t rows, int64_t dim) {
     dep_trigger();
     dep_wait();
-    const int lane = threadIdx.x & 31;
-    const int64_t row = (int64_t)blockIdx.x * NORM_WARPS + (threadIdx.x >> 5);
-    if (row >= rows) return;
-    const int nvec = (int)(dim / 8);
-    float v[VPL][8];
+    __shared__ float s0[ROW_SLOTS], s1[ROW_SLOTS];
+    const int i = threadIdx.x * 8;
+    const int64_t row = (int64_t)blockIdx.x * blockDim.y + threadIdx.y, at = row * dim + i;
+    const bool in = row < rows && i < dim;
+    float v[8], r[8], wp[8], wn[8];
+    zero8(v); zero8(r); zero8(wp); zero8(wn);
+    if (in) {
+        load8(y + at, v);
+        load8(residual + at, r);
+        load8(w_post + i, wp);
+        load8(w_next + i, wn);
+    }
     float ss = 0.f;
 #pragma unroll
-    for (int k = 0; k < VPL; ++k) {
-        const int i = lane + k * 32;
-        if (i < nvec) load8(y + row * dim + i * 8, v[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < VPL; ++k) {
-        const int i = lane + k * 32;
-        if (i < nvec) prefetch_l1(residual + row * dim + i * 8);
-    }
-#pragma unroll
-    for (int k = 0; k < VPL; ++k)
-        if (lane + k * 32 < nvec) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) ss += v[k][j] * v[k][j];
-        }
-    ss = warp_sum(ss);
+    for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
+    ss = row_sum(ss, s0);
     const float rp = rsqrtf(ss / (float)dim + eps);
-    if (lane == 0) rstd_post[row] = rp;
+    if (threadIdx.x == 0 && in) rstd_post[row] = rp;
     float ss2 = 0.f;
 #pragma unroll
-    for (int k = 0; k < VPL; ++k) {
-        const int i = lane + k * 32;
-        if (i < nvec) {
-            float wv[8], r[8];
-            load8(w_post + i * 8, wv);
-            load8(residual + row * dim + i * 8, r);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float o = v[k][j] * rp * (unit_post ? 1.0f + wv[j] : wv[j]);
-                v[k][j] = r[j] + o;
-            }
-            store8(sum_out + row * dim + i * 8, v[k]);
-        }
+    for (int j = 0; j < 8; ++j) {
+        v[j] = __fadd_rn(r[j], norm_out(v[j], rp, unit_post ? 1.0f + wp[j] : wp[j]));
+        ss2 += v[j] * v[j];
     }
-#pragma unroll
-    for (int k = 0; k < VPL; ++k)
-        if (lane + k * 32 < nvec) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) ss2 += v[k][j] * v[k][j];
-        }
-    ss2 = warp_sum(ss2);
+    if (in) store8(sum_out + at, v);
+    ss2 = row_sum(ss2, s1);
     const float rn = rsqrtf(ss2 / (float)dim + eps);
-    if (lane == 0) rstd_next[row] = rn;
+    if (threadIdx.x == 0 && in) rstd_next[row] = rn;
+    if (!in) return;
+    float o[8];
 #pragma unroll
-    for (int k = 0; k < VPL; ++k) {
-        const int i = lane + k * 32;
-        if (i < nvec) {
-            float wv[8], o[8];
-            load8(w_next + i * 8, wv);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] = v[k][j] * rn * (unit_next ? 1.0f + wv[j] : wv[j]);
-            store8(h_next + row * dim + i * 8, o);
-        }
-    }
+    for (int j = 0; j < 8; ++j) o[j] = norm_out(v[j], rn, unit_next ? 1.0f + wn[j] : wn[j]);
+    store8(h_next + at, o);
 }
 
 // Backward of the same pair: dx (f32, the gradient on x_sum that came down the residual path) first receives the
 // gradient through the next pre-norm (dy_next), is stored, and then goes through the post-norm of the branch.
-template <int VPL>
-__global__ void __launch_bounds__(NORM_WARPS * 32)
-rmsnorm_pair_bwd_kernel(const __nv_bfloat16* __restrict__ dy_next, const float* __restrict__ x_sum, const float* __restrict__ w_next,
+__global__ void __launch_bounds__(ROW_MAX_WARPS * 32)
+rmsnorm_pair_bwd_kernel(const __nv_bfloat16* dy_next, const float* __restrict__ x_sum, const float* __restrict__ w_next,
                         int unit_next, const float* __restrict__ rstd_next, float* __restrict__ dx,
                         const __nv_bfloat16* __restrict__ y_branch, const float* __restrict__ w_post, int unit_post,
-                        const float* __restrict__ rstd_post, __nv_bfloat16* __restrict__ d_branch, int64_t rows, int64_t dim) {
+                        const float* __restrict__ rstd_post, __nv_bfloat16* d_branch, int64_t rows, int64_t dim) {
+    // d_branch may be dy_next: a thread reads its columns before it writes them and no other thread touches them
     dep_trigger();
     dep_wait();
-    const int lane = threadIdx.x & 31;
-    const int64_t row = (int64_t)blockIdx.x * NORM_WARPS + (threadIdx.x >> 5);
-    if (row >= rows) return;
-    const int nvec = (int)(dim / 8);
-    float xv[VPL][8], g[VPL][8];
-#pragma unroll
-    for (int k = 0; k < VPL; ++k) {
-        const int i = lane + k * 32;
-        if (i < nvec) {
-            load8(x_sum + row * dim + i * 8, xv[k]);
-            load8(dy_next + row * dim + i * 8, g[k]);
-        }
+    __shared__ float s0[ROW_SLOTS], s1[ROW_SLOTS];
+    const int i = threadIdx.x * 8;
+    const int64_t row = (int64_t)blockIdx.x * blockDim.y + threadIdx.y, at = row * dim + i;
+    const bool in = row < rows && i < dim;
+    float xv[8], g[8], prev[8], yv[8], wn[8], wp[8];
+    zero8(xv); zero8(g); zero8(prev); zero8(yv); zero8(wn); zero8(wp);
+    if (in) {
+        load8(x_sum + at, xv);
+        load8(dy_next + at, g);
+        load8(dx + at, prev);
+        load8(y_branch + at, yv);
+        load8(w_next + i, wn);
+        load8(w_post + i, wp);
     }
-#pragma unroll
-    for (int k = 0; k < VPL; ++k) {
-        const int i = lane + k * 32;
-        if (i < nvec) {
-            prefetch_l1(dx + row * dim + i * 8);
-            if ((i & 1) == 0) prefetch_l1(y_branch + row * dim + i * 8);      // 16-byte pieces: every other lane names a new 32 bytes
-        }
-    }
+    const float rn = row < rows ? rstd_next[row] : 0.f, rp = row < rows ? rstd_post[row] : 0.f;
     float dot = 0.f;
 #pragma unroll
-    for (int k = 0; k < VPL; ++k) {
-        const int i = lane + k * 32;
-        if (i < nvec) {
-            float wv[8];
-            load8(w_next + i * 8, wv);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                g[k][j] *= (unit_next ? 1.0f + wv[j] : wv[j]);
-                dot += g[k][j] * xv[k][j];
-            }
-        }
+    for (int j = 0; j < 8; ++j) {
+        g[j] *= (unit_next ? 1.0f + wn[j] : wn[j]);
+        dot += g[j] * xv[j];
     }
-    dot = warp_sum(dot);
-    const float rn = rstd_next[row];
+    dot = row_sum(dot, s0);
     const float coeff = rn * rn * rn / (float)dim * dot;
-#pragma unroll
-    for (int k = 0; k < VPL; ++k) {
-        const int i = lane + k * 32;
-        if (i < nvec) {
-            float prev[8];
-            load8(dx + row * dim + i * 8, prev);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) g[k][j] = (g[k][j] * rn - xv[k][j] * coeff) + prev[j];
-            store8(dx + row * dim + i * 8, g[k]);
-        }
-    }
     // post-norm of the branch: dy = the dx row just formed
-    float dot2 = 0.f;
+    float dot2 = 0.f, dxv[8];
 #pragma unroll
-    for (int k = 0; k < VPL; ++k) {
-        const int i = lane + k * 32;
-        if (i < nvec) {
-            float wv[8];
-            load8(y_branch + row * dim + i * 8, xv[k]);
-            load8(w_post + i * 8, wv);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                g[k][j] *= (unit_post ? 1.0f + wv[j] : wv[j]);
-                dot2 += g[k][j] * xv[k][j];
-            }
-        }
+    for (int j = 0; j < 8; ++j) {
+        dxv[j] = __fadd_rn(norm_grad(g[j], rn, xv[j], coeff), prev[j]);
+        g[j] = dxv[j] * (unit_post ? 1.0f + wp[j] : wp[j]);
+        dot2 += g[j] * yv[j];
     }
-    dot2 = warp_sum(dot2);
-    const float rp = rstd_post[row];
+    if (in) store8(dx + at, dxv);
+    dot2 = row_sum(dot2, s1);
     const float coeff2 = rp * rp * rp / (float)dim * dot2;
+    if (!in) return;
+    float o[8];
 #pragma unroll
-    for (int k = 0; k < VPL; ++k) {
-        const int i = lane + k * 32;
-        if (i < nvec) {
-            float o[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] = g[k][j] * rp - xv[k][j] * coeff2;
-            store8(d_branch + row * dim + i * 8, o);
-        }
-    }
+    for (int j = 0; j < 8; ++j) o[j] = norm_grad(g[j], rp, yv[j], coeff2);
+    store8(d_branch + at, o);
 }
 
 // ---------------------------------------------------------------- LayerNorm
@@ -727,15 +655,11 @@ int32_t mft_rmsnorm_fwd(const void* x, int32_t xd, const float* w, float eps, in
     MFT_CHECK_ARG(y || (residual && sum_out), "mft_rmsnorm_fwd: nothing to write");
     MFT_CHECK_ARG(!residual || sum_out, "mft_rmsnorm_fwd: residual needs sum_out");
     MFT_CHECK_ARG(dim % 8 == 0 && dim <= 8 * NORM_THREADS * NORM_VPT, "mft_rmsnorm_fwd: dim must be a multiple of 8 and <= 4096");
-    const unsigned wblocks = (unsigned)((rows + NORM_WARPS - 1) / NORM_WARPS);
-#define WCALL(TX, TY, VPL) launch_dep(rmsnorm_fwd_warp_kernel<TX, TY, VPL>, dim3(wblocks), dim3(NORM_WARPS * 32), (size_t)(0), as_stream(stream), (const TX*)x, w, eps, unit_offset, (TY*)y, rstd, residual, sum_out, rows, dim);
 #define CALL(TX, TY)                                                                                     \
-    if (dim <= 1280) { WCALL(TX, TY, 5) }                                                                \
-    else if (dim <= 2048) { WCALL(TX, TY, 8) }                                                           \
+    if (dim <= ROW_MAX_DIM) launch_dep(rmsnorm_fwd_row_kernel<TX, TY>, row_grid(rows, dim), row_block(dim), (size_t)(0), as_stream(stream), (const TX*)x, w, eps, unit_offset, (TY*)y, rstd, residual, sum_out, rows, dim); \
     else launch_dep(rmsnorm_fwd_kernel<TX, TY>, dim3((unsigned)rows), dim3(NORM_THREADS), (size_t)(0), as_stream(stream), (const TX*)x, w, eps, unit_offset, (TY*)y, rstd, residual, sum_out, dim);
     DISPATCH_2(xd, yd, CALL)
 #undef CALL
-#undef WCALL
     MFT_LAUNCH_CHECK("rmsnorm_fwd");
     return MFT_OK;
 }
@@ -747,17 +671,13 @@ int32_t mft_rmsnorm_bwd(const void* dy, int32_t dyd, const void* x, int32_t xd, 
     MFT_CHECK_ARG(dim % 8 == 0 && dim <= 8 * NORM_THREADS * NORM_VPT, "mft_rmsnorm_bwd: dim must be a multiple of 8 and <= 4096");
     MFT_CHECK_ARG(!accumulate || dxd == MFT_F32, "mft_rmsnorm_bwd: accumulate needs f32 dx");
     MFT_CHECK_ARG(!dweight || rstd, "mft_rmsnorm_bwd: dweight needs rstd");
-    const unsigned wblocks = (unsigned)((rows + NORM_WARPS - 1) / NORM_WARPS);
-#define WLAUNCH(TDY, TX, TDX, VPL) launch_dep(rmsnorm_bwd_warp_kernel<TDY, TX, TDX, VPL>, dim3(wblocks), dim3(NORM_WARPS * 32), (size_t)(0), as_stream(stream), (const TDY*)dy, (const TX*)x, w, rstd, eps, unit_offset, (TDX*)dx, accumulate, dweight, rows, dim);
 #define LAUNCH(TDY, TX, TDX)                                                                             \
-    if (dim <= 1280) { WLAUNCH(TDY, TX, TDX, 5) }                                                        \
-    else if (dim <= 2048) { WLAUNCH(TDY, TX, TDX, 8) }                                                   \
+    if (dim <= ROW_MAX_DIM) launch_dep(rmsnorm_bwd_row_kernel<TDY, TX, TDX>, row_grid(rows, dim), row_block(dim), (size_t)(0), as_stream(stream), (const TDY*)dy, (const TX*)x, w, rstd, eps, unit_offset, (TDX*)dx, accumulate, dweight, rows, dim); \
     else launch_dep(rmsnorm_bwd_kernel<TDY, TX, TDX>, dim3((unsigned)rows), dim3(NORM_THREADS), (size_t)(0), as_stream(stream), (const TDY*)dy, (const TX*)x, w, rstd, eps, unit_offset, (TDX*)dx, accumulate, dweight, dim);
 #define CALL(TDY, TX) if (dxd == MFT_F32) { LAUNCH(TDY, TX, float) } else if (dxd == MFT_BF16) { LAUNCH(TDY, TX, __nv_bfloat16) } else return fail(MFT_ERR_INVALID_ARG, "mft_rmsnorm_bwd: bad dx dtype");
     DISPATCH_2(dyd, xd, CALL)
 #undef CALL
 #undef LAUNCH
-#undef WLAUNCH
     MFT_LAUNCH_CHECK("rmsnorm_bwd");
     return MFT_OK;
 }
@@ -767,13 +687,10 @@ int32_t mft_rmsnorm_add_norm_fwd(const void* y_bf16, const float* w_post, int32_
                                  void* h_next_bf16, float* rstd_next, int64_t rows, int64_t dim, mft_stream_t stream) {
     MFT_CHECK_ARG(y_bf16 && w_post && residual && w_next && sum_out && rstd_post && h_next_bf16 && rstd_next && rows > 0, "mft_rmsnorm_add_norm_fwd: bad argument");
     MFT_CHECK_ARG(dim > 0 && dim % 8 == 0, "mft_rmsnorm_add_norm_fwd: dim must be a multiple of 8");
-    if (dim > 2048) return fail(MFT_ERR_UNSUPPORTED, "mft_rmsnorm_add_norm_fwd: rows wider than 2048 use the separate norm calls");
-    const unsigned wblocks = (unsigned)((rows + NORM_WARPS - 1) / NORM_WARPS);
-#define FCALL(VPL) launch_dep(rmsnorm_add_norm_fwd_kernel<VPL>, dim3(wblocks), dim3(NORM_WARPS * 32), (size_t)0, as_stream(stream), \
-                              (const __nv_bfloat16*)y_bf16, w_post, (int)unit_post, residual, w_next, (int)unit_next, eps, sum_out, rstd_post, \
-                              (__nv_bfloat16*)h_next_bf16, rstd_next, rows, dim)
-    if (dim <= 1280) FCALL(5); else FCALL(8);
-#undef FCALL
+    if (dim > ROW_MAX_DIM) return fail(MFT_ERR_UNSUPPORTED, "mft_rmsnorm_add_norm_fwd: rows wider than 2048 use the separate norm calls");
+    launch_dep(rmsnorm_add_norm_fwd_kernel, row_grid(rows, dim), row_block(dim), (size_t)0, as_stream(stream),
+               (const __nv_bfloat16*)y_bf16, w_post, (int)unit_post, residual, w_next, (int)unit_next, eps, sum_out, rstd_post,
+               (__nv_bfloat16*)h_next_bf16, rstd_next, rows, dim);
     MFT_LAUNCH_CHECK("rmsnorm_add_norm_fwd");
     return MFT_OK;
 }
@@ -785,13 +702,10 @@ int32_t mft_rmsnorm_pair_bwd(const void* dy_next_bf16, const float* x_sum, const
     MFT_CHECK_ARG(dy_next_bf16 && x_sum && w_next && rstd_next && dx_inout && y_branch_bf16 && w_post && rstd_post && d_branch_bf16 && rows > 0,
                   "mft_rmsnorm_pair_bwd: bad argument");
     MFT_CHECK_ARG(dim > 0 && dim % 8 == 0, "mft_rmsnorm_pair_bwd: dim must be a multiple of 8");
-    if (dim > 2048) return fail(MFT_ERR_UNSUPPORTED, "mft_rmsnorm_pair_bwd: rows wider than 2048 use the separate norm calls");
-    const unsigned wblocks = (unsigned)((rows + NORM_WARPS - 1) / NORM_WARPS);
-#define BCALL(VPL) launch_dep(rmsnorm_pair_bwd_kernel<VPL>, dim3(wblocks), dim3(NORM_WARPS * 32), (size_t)0, as_stream(stream), \
-                              (const __nv_bfloat16*)dy_next_bf16, x_sum, w_next, (int)unit_next, rstd_next, dx_inout, \
-                              (const __nv_bfloat16*)y_branch_bf16, w_post, (int)unit_post, rstd_post, (__nv_bfloat16*)d_branch_bf16, rows, dim)
-    if (dim <= 1280) BCALL(5); else BCALL(8);
-#undef BCALL
+    if (dim > ROW_MAX_DIM) return fail(MFT_ERR_UNSUPPORTED, "mft_rmsnorm_pair_bwd: rows wider than 2048 use the separate norm calls");
+    launch_dep(rmsnorm_pair_bwd_kernel, row_grid(rows, dim), row_block(dim), (size_t)0, as_stream(stream),
+               (const __nv_bfloat16*)dy_next_bf16, x_sum, w_next, (int)unit_next, rstd_next, dx_inout,
+               (const __nv_bfloat16*)y_branch_bf16, w_post, (int)unit_post, rstd_post, (__nv_bfloat16*)d_branch_bf16, rows, dim);
     MFT_LAUNCH_CHECK("rmsnorm_pair_bwd");
     return MFT_OK;
 }
