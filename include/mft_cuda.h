@@ -321,7 +321,8 @@ int32_t mft_glu_linear_bwd(int32_t kind, const void* dy_bf16, int64_t lddy, cons
  * any other even head_dim <= 256 on generic kernels, all with the same results
  * to bf16 rounding.  MFT_ATTN_TC=0 in the environment selects the mma.sync
  * kernels everywhere, MFT_ATTN_TC=2 the tensor-memory kernels at every shape
- * they take. */
+ * they take.  Strides are multiples of 8 elements; q, k, v, d_o start on 16 bytes, o, dq, dk, dv on 4 (the
+ * tensor-memory kernels store 16 bytes at a time and leave outputs that start elsewhere to the mma.sync kernels). */
 typedef struct {
     int64_t stride_b, stride_s, stride_h;
 } mft_strides_t;

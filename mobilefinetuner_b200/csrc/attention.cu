@@ -648,6 +648,10 @@ extern "C" int32_t mft_attn_bwd(const void* q, mft_strides_t sq, const void* k, 
     // mma.sync CTA per query head when a KV group has several heads (more, shorter CTAs)
     const int shape = attn_shape_override();
     bool dkv_tc = false;
+    // attn_dkv_store_kernel reads the scratch in 16-byte and writes dK / dV in 8-byte words; anywhere else than on such
+    // addresses the kernel without scratch takes the call (its stores are 4 bytes)
+    auto on = [](const void* q, uintptr_t bytes) { return reinterpret_cast<uintptr_t>(q) % bytes == 0; };
+    if (!on(dkv_acc, 16) || !on(dk, 8) || !on(dv, 8)) p.dkv_acc = dkv_acc = nullptr;
     if (dkv_acc != nullptr)
         if (int32_t s = check_cuda(cudaMemsetAsync(dkv_acc, 0, (size_t)(2 * batch * seq * n_kv * hd) * sizeof(float), as_stream(stream)), "attention dkv memset")) return s;
     const bool split = dkv_acc != nullptr && p.rep > 1;

@@ -961,6 +961,9 @@ attn_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 
 bool token_major(const mft_strides_t& s, int seq) { return s.stride_b == (int64_t)seq * s.stride_s; }
 
+// The epilogues store 16 bytes at a time (the mma.sync kernels 4): strides are multiples of 8 elements, so the base decides
+bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
+
 bool tc_shape_ok(int hd) { return hd == 64 || hd == 128 || hd == 256; }
 
 template <int HD>
@@ -1031,6 +1034,7 @@ int32_t attn_fwd_sm100(const AttnParams& a, int hd, cudaStream_t stream) {
     if (a.seq <= (hd == 256 ? 256 : hd == 128 ? 128 : 384) && enabled < 2) return MFT_ERR_UNSUPPORTED;
     if (!token_major(a.sq, a.seq) || !token_major(a.sk, a.seq) || !token_major(a.sv, a.seq)) return MFT_ERR_UNSUPPORTED;
     if (a.sq.stride_h % 8 || a.sk.stride_h % 8 || a.sv.stride_h % 8 || a.so.stride_s % 8 || a.so.stride_h % 8 || a.so.stride_b % 8) return MFT_ERR_UNSUPPORTED;
+    if (!aligned16(a.out)) return MFT_ERR_UNSUPPORTED;
     if ((int64_t)a.batch * a.seq >= (1ll << 31)) return MFT_ERR_UNSUPPORTED;
     CUtensorMap mq, mk, mv;
     if (make_tmap_bf16_batched(&mq, a.q, a.batch, a.seq, (int64_t)(a.n_heads - 1) * a.sq.stride_h + hd, a.sq.stride_s, BM) != MFT_OK) return MFT_ERR_UNSUPPORTED;
@@ -1051,6 +1055,7 @@ int32_t attn_dq_sm100(const AttnParams& a, int hd, bool compute_delta, cudaStrea
     if (!enabled || !tc_shape_ok(hd) || !device_status_word()) return MFT_ERR_UNSUPPORTED;
     if (!bwd_long_enough(hd, a.seq) && enabled < 2) return MFT_ERR_UNSUPPORTED;
     if (compute_delta && hd != 256) return MFT_ERR_UNSUPPORTED;
+    if (!aligned16(a.dq)) return MFT_ERR_UNSUPPORTED;
     if (!token_major(a.sq, a.seq) || !token_major(a.sk, a.seq) || !token_major(a.sv, a.seq) || !token_major(a.sdo, a.seq)) return MFT_ERR_UNSUPPORTED;
     if (a.sq.stride_h % 8 || a.sk.stride_h % 8 || a.sv.stride_h % 8 || a.sdo.stride_h % 8) return MFT_ERR_UNSUPPORTED;
     if ((int64_t)a.batch * a.seq >= (1ll << 31)) return MFT_ERR_UNSUPPORTED;
@@ -1082,7 +1087,7 @@ int32_t attn_dkv_sm100(const AttnParams& a, int hd, cudaStream_t stream) {
     if (!token_major(a.sq, a.seq) || !token_major(a.sk, a.seq) || !token_major(a.sv, a.seq) || !token_major(a.sdo, a.seq)) return MFT_ERR_UNSUPPORTED;
     if (a.sq.stride_h % 8 || a.sk.stride_h % 8 || a.sv.stride_h % 8 || a.sdo.stride_h % 8) return MFT_ERR_UNSUPPORTED;
     if ((int64_t)a.batch * a.seq >= (1ll << 31) || 2 * a.n_heads > 65535) return MFT_ERR_UNSUPPORTED;
-    if (reinterpret_cast<uintptr_t>(a.lse) % 16 || reinterpret_cast<uintptr_t>(a.delta) % 16 || reinterpret_cast<uintptr_t>(a.dkv_acc) % 16) return MFT_ERR_UNSUPPORTED;
+    if (!aligned16(a.lse) || !aligned16(a.delta) || !aligned16(a.dkv_acc)) return MFT_ERR_UNSUPPORTED;
     CUtensorMap mq, md, mk, mv;
     if (make_tmap_bf16_batched(&mq, a.q, a.batch, a.seq, (int64_t)(a.n_heads - 1) * a.sq.stride_h + hd, a.sq.stride_s, KV_BQ) != MFT_OK) return MFT_ERR_UNSUPPORTED;
     if (make_tmap_bf16_batched(&md, a.d_o, a.batch, a.seq, (int64_t)(a.n_heads - 1) * a.sdo.stride_h + hd, a.sdo.stride_s, KV_BQ) != MFT_OK) return MFT_ERR_UNSUPPORTED;

@@ -47,3 +47,37 @@ def test_ragged_sequences(hd, heads, kv, seq, window):
         row = (a - b).norm(dim=-1) if a.dim() == 4 else (a - b).abs()
         size = b.norm(dim=-1) if a.dim() == 4 else b.abs()
         assert (row <= 2 ** -5 * (size + size.mean())).all(), name
+
+
+# the mma.sync kernels store 4 bytes at a time and take outputs that start on any 4 bytes; the tensor-memory kernels do not
+@pytest.mark.parametrize("hd,heads,kv,seq", [(64, 14, 2, 401), (64, 4, 4, 512), (128, 4, 4, 201), (128, 4, 2, 1000), (256, 4, 1, 300), (256, 2, 2, 384)])
+@pytest.mark.parametrize("shift", [2, 4])       # elements of 2 bytes that the outputs start after a 16-byte boundary
+def test_outputs_off_16_bytes(hd, heads, kv, seq, shift):
+    from mobilefinetuner_b200 import _lib as L
+    from mobilefinetuner_b200 import ops as O
+    b = 2
+    g = torch.Generator(device="cuda").manual_seed(seq + shift)
+
+    def rnd(n):
+        return torch.randn(b, seq, n, hd, device="cuda", generator=g).bfloat16().permute(0, 2, 1, 3)
+
+    def off(n):
+        buf = torch.full((b * seq * n * hd + 8,), float("nan"), device="cuda").bfloat16()
+        return buf[shift:shift + b * seq * n * hd].view(b, seq, n, hd).permute(0, 2, 1, 3), buf
+    q, k, v, d_o = rnd(heads), rnd(kv), rnd(kv), rnd(heads)
+    (o, o_buf), (dq, dq_buf), (dk, dk_buf), (dv, dv_buf) = off(heads), off(heads), off(kv), off(kv)
+    lse, delta = torch.empty(b, heads, seq, device="cuda"), torch.empty(b, heads, seq, device="cuda")
+    acc = torch.empty(2 * b * seq * kv * hd, device="cuda")
+    scale, st = hd ** -0.5, torch.cuda.current_stream().cuda_stream
+    L.init(0)
+
+    def ps(*ts):
+        return [x for t in ts for x in (t.data_ptr(), O._strides_bhsd(t))]
+    L.call("mft_attn_fwd", *ps(q, k, v, o), lse.data_ptr(), b, seq, heads, kv, hd, scale, 0, st)
+    L.call("mft_attn_bwd", *ps(q, k, v, o, d_o), lse.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), delta.data_ptr(), acc.data_ptr(),
+           b, seq, heads, kv, hd, scale, 0, st)
+    ref = _reference(q, k, v, d_o, scale, 0)
+    for name, x, r in zip(("o", "lse", "dq", "dk", "dv"), (o, lse, dq, dk, dv), ref):
+        assert (x.float() - r).norm() <= 2 ** -7 * r.norm(), name       # as above
+    for buf in (o_buf, dq_buf, dk_buf, dv_buf):
+        assert bool(buf[:shift].isnan().all()) and bool(buf[buf.numel() - 8 + shift:].isnan().all())
