@@ -16,7 +16,8 @@
 // than 2^8 since the last rescale, which keeps the exponentials below 256 and makes rescales rare.
 // Sequences of any length: the tensor maps are [batch, sequence, columns], so that a tile's rows past the end of a sequence
 // read as zeros (never as the next sample), and only stores look at the length; the causal mask hides keys past the end from
-// every row that is stored.  At 3 x 1001 tokens, 4 / 1 heads of 256, forward / dQ / dK + dV took 54 / 89 / 87 us on the
+// every row that is stored.  (The backward kernels keep [batch * sequence, columns] maps for sequences of whole tiles, see
+// launch_dq; the forward measured 1 to 3 % faster with the three-dimensional ones at every length.)  At 3 x 1001 tokens, 4 / 1 heads of 256, forward / dQ / dK + dV took 54 / 89 / 87 us on the
 // mma.sync kernels; the whole backward is 125 instead of 274 us at 4 x 1001.
 // Every mbarrier wait is bounded; a wait that runs out sets the library status word and the CTA leaves.
 #include <cuda.h>
@@ -105,6 +106,30 @@ __device__ __forceinline__ uint64_t smem_desc_mn_sw128(uint32_t smem_addr, uint3
 // Wait of a whole MMA-issuing warp: the warp stays converged, one elected lane issues (see the pair GEMM's issuer)
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)) != 0;
+}
+// Issuing form of the backward kernels.  WARP: the warp stays converged and one elected lane issues.  Otherwise lane 0 walks
+// the loop alone, which at head_dim 256 is 1 to 2 % of the whole backward pass faster (4 x 1001 tokens, 4 / 1 heads, window
+// 512: 108.7 against 107.3 us), at 64 2.5 % slower (8 x 4096, 14 / 2 heads: 1730 against 1775) and at 128 1 % (1714 / 1733).
+template <bool WARP>
+struct Issue {
+    static __device__ __forceinline__ bool joins(int lane) { return WARP || lane == 0; }
+    static __device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+        if constexpr (WARP) return warp_wait(bar, parity, abort_flag);
+        else return mbar_wait(bar, parity, abort_flag);
+    }
+    static __device__ __forceinline__ bool elected() {
+        if constexpr (WARP) return elect_one();
+        else return true;
+    }
+    static __device__ __forceinline__ void done() { if constexpr (WARP) __syncwarp(); }
+};
+// One box of the backward kernels: rows from `row` on of sample b.  RAGGED: the tensor map is [batch, sequence, columns], so
+// that a box's rows past the end of the sequence read as zeros.  Otherwise it is [batch * sequence, columns], for sequences
+// of whole 128-row tiles (see launch_dq for what the two cost).
+template <bool RAGGED>
+__device__ __forceinline__ void load_box(void* dst, const CUtensorMap* map, uint64_t* bar, int col, int row, int b, int seq) {
+    if constexpr (RAGGED) tma_load_3d(dst, map, bar, col, row, b);
+    else tma_load_2d(dst, map, bar, col, b * seq + row);
 }
 constexpr uint32_t IDESC_B_MN = 1u << 16;      // instruction-descriptor bit: B operand is MN-major
 
@@ -432,7 +457,7 @@ struct BwdParams {
     float* delta_out;
 };
 
-template <int HD>
+template <int HD, bool RAGGED>
 __global__ void __launch_bounds__(DqDim<HD>::THREADS, DqDim<HD>::GROUPS == 1 ? 2 : 1)
 attn_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
                   const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const BwdParams p) {
@@ -467,7 +492,7 @@ attn_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     const int h = blockIdx.y, b = blockIdx.z;
     const int kvh = h / p.rep;
     const int i0 = qb * BM;
-    const int jb_hi = (min(i0 + BM, p.seq) - 1) / DQ_BN;
+    const int jb_hi = ((RAGGED ? min(i0 + BM, p.seq) : i0 + BM) - 1) / DQ_BN;
     const int jb_lo = p.window > 0 ? max(0, i0 - p.window + 1) / DQ_BN : 0;
     const int n_tiles = jb_hi - jb_lo + 1;
 
@@ -493,68 +518,70 @@ attn_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     if (warp == 0) {
         if (lane == 0) {
             mbar_arrive_expect_tx(qdo_full, 2 * Q_BYTES);
-            for (int c = 0; c < CH; ++c) tma_load_3d(q_smem + c * (BM * 128), &map_q, qdo_full, h * p.q_col0_stride + c * 64, i0, b);
-            for (int c = 0; c < CH; ++c) tma_load_3d(do_smem + c * (BM * 128), &map_do, qdo_full, h * p.do_col0_stride + c * 64, i0, b);
+            for (int c = 0; c < CH; ++c) load_box<RAGGED>(q_smem + c * (BM * 128), &map_q, qdo_full, h * p.q_col0_stride + c * 64, i0, b, p.seq);
+            for (int c = 0; c < CH; ++c) load_box<RAGGED>(do_smem + c * (BM * 128), &map_do, qdo_full, h * p.do_col0_stride + c * 64, i0, b, p.seq);
             for (int t = 0; t < n_tiles; ++t) {
                 const int ks = t % DQ_KST, vs = t & 1;
                 const uint32_t kph = (t / DQ_KST) & 1, vph = (t >> 1) & 1;
                 const int row = (jb_lo + t) * DQ_BN;
                 if (!mbar_wait(&k_empty[ks], kph ^ 1, abort_flag)) break;
                 mbar_arrive_expect_tx(&k_full[ks], DQ_KV_BYTES);
-                for (int c = 0; c < CH; ++c) tma_load_3d(k_smem + ks * DQ_KV_BYTES + c * (DQ_BN * 128), &map_k, &k_full[ks], kvh * p.k_col0_stride + c * 64, row, b);
+                for (int c = 0; c < CH; ++c) load_box<RAGGED>(k_smem + ks * DQ_KV_BYTES + c * (DQ_BN * 128), &map_k, &k_full[ks], kvh * p.k_col0_stride + c * 64, row, b, p.seq);
                 if (!mbar_wait(&v_empty[vs], vph ^ 1, abort_flag)) break;
                 mbar_arrive_expect_tx(&v_full[vs], DQ_KV_BYTES);
-                for (int c = 0; c < CH; ++c) tma_load_3d(v_smem + vs * DQ_KV_BYTES + c * (DQ_BN * 128), &map_v, &v_full[vs], kvh * p.v_col0_stride + c * 64, row, b);
+                for (int c = 0; c < CH; ++c) load_box<RAGGED>(v_smem + vs * DQ_KV_BYTES + c * (DQ_BN * 128), &map_v, &v_full[vs], kvh * p.v_col0_stride + c * 64, row, b, p.seq);
             }
         }
     } else if (warp == 1 || warp == W_DP) {
         // ------------------------------------------------ MMA issuers 1 and 2: S = Q K^T (warp 1), dP = dO V^T (warp W_DP)
-        {
+        using I = Issue<HD != 256>;
+        if (I::joins(lane)) {
             constexpr uint32_t idesc_s = idesc_bf16_f32(BM, DQ_BN);
             const bool is_s = warp == 1;
-            bool ok = warp_wait(qdo_full, 0, abort_flag);
+            bool ok = I::wait(qdo_full, 0, abort_flag);
             const uint64_t ad = smem_desc_sw128(smem_u32(is_s ? q_smem : do_smem));
             for (int t = 0; t < n_tiles && ok; ++t) {
                 const int g = t & 1, ks = t % DQ_KST;
                 const uint32_t gph = (t >> 1) & 1, kph = (t / DQ_KST) & 1;
-                if (!warp_wait(is_s ? &k_full[ks] : &v_full[g], is_s ? kph : gph, abort_flag)) { ok = false; break; }
-                if (!warp_wait(&sdp_free[g], gph ^ 1, abort_flag)) { ok = false; break; }
+                if (!I::wait(is_s ? &k_full[ks] : &v_full[g], is_s ? kph : gph, abort_flag)) { ok = false; break; }
+                if (!I::wait(&sdp_free[g], gph ^ 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
-                if (elect_one()) {
-                const uint64_t bd = smem_desc_sw128(smem_u32(is_s ? k_smem + ks * DQ_KV_BYTES : v_smem + g * DQ_KV_BYTES));
-                const uint32_t tmem_d = tmem_base + (is_s ? DQ_S_COL : DQ_DP_COL) + g * DQ_BN;
+                if (I::elected()) {
+                    const uint64_t bd = smem_desc_sw128(smem_u32(is_s ? k_smem + ks * DQ_KV_BYTES : v_smem + g * DQ_KV_BYTES));
+                    const uint32_t tmem_d = tmem_base + (is_s ? DQ_S_COL : DQ_DP_COL) + g * DQ_BN;
 #pragma unroll
-                for (int c = 0; c < CH; ++c)
+                    for (int c = 0; c < CH; ++c)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        umma_bf16(tmem_d, ad + (uint64_t)(c * (BM * 128 / 16) + 2 * j), bd + (uint64_t)(c * (DQ_BN * 128 / 16) + 2 * j), idesc_s,
-                                  (c | j) != 0 ? 1u : 0u);
-                if (!is_s) umma_commit(&v_empty[g]);
-                umma_commit(&sdp_full[g]);            // two arrivals complete it: S and dP
+                        for (int j = 0; j < 4; ++j)
+                            umma_bf16(tmem_d, ad + (uint64_t)(c * (BM * 128 / 16) + 2 * j), bd + (uint64_t)(c * (DQ_BN * 128 / 16) + 2 * j), idesc_s,
+                                      (c | j) != 0 ? 1u : 0u);
+                    if (!is_s) umma_commit(&v_empty[g]);
+                    umma_commit(&sdp_full[g]);            // two arrivals complete it: S and dP
                 }
-                __syncwarp();
+                I::done();
             }
         }
     } else if (warp == W_DQ) {
         // ------------------------------------------------ MMA issuer 3: dQ += dS K
-        {
+        using I = Issue<HD != 256>;
+        if (I::joins(lane)) {
             constexpr uint32_t idesc_acc = idesc_bf16_f32(BM, HD) | IDESC_B_MN;
             bool ok = true;
             for (int t = 0; t < n_tiles && ok; ++t) {
                 const int g = t & 1, ks = t % DQ_KST;
                 const uint32_t gph = (t >> 1) & 1;
-                if (!warp_wait(&ds_full[g], gph, abort_flag)) { ok = false; break; }
+                if (!I::wait(&ds_full[g], gph, abort_flag)) { ok = false; break; }
                 tc_fence_after();
-                if (elect_one()) {
-                const uint64_t kd = smem_desc_mn_sw128(smem_u32(k_smem + ks * DQ_KV_BYTES), DQ_BN * 128);
+                if (I::elected()) {
+                    const uint64_t kd = smem_desc_mn_sw128(smem_u32(k_smem + ks * DQ_KV_BYTES), DQ_BN * 128);
 #pragma unroll
-                for (int j = 0; j < 2; ++j)
-                    umma_bf16_ts(tmem_base + DQ_ACC_COL, tmem_base + DQ_DS_COL + g * 16 + 8 * j, kd + (uint64_t)(j * (2048 / 16)), idesc_acc, (t | j) != 0 ? 1u : 0u);
-                umma_commit(&k_empty[ks]);
-                umma_commit(&ds_free[g]);
-                if (t == n_tiles - 1) umma_commit(acc_done);
+                    for (int j = 0; j < 2; ++j)
+                        umma_bf16_ts(tmem_base + DQ_ACC_COL, tmem_base + DQ_DS_COL + g * 16 + 8 * j, kd + (uint64_t)(j * (2048 / 16)), idesc_acc, (t | j) != 0 ? 1u : 0u);
+                    umma_commit(&k_empty[ks]);
+                    umma_commit(&ds_free[g]);
+                    if (t == n_tiles - 1) umma_commit(acc_done);
                 }
-                __syncwarp();
+                I::done();
             }
         }
     } else {
@@ -565,7 +592,7 @@ attn_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         const int i = i0 + r;
         const uint32_t lane_addr = tmem_base + ((uint32_t)(q4 * 32) << 16);
         const float sl2 = p.scale * LOG2E;
-        const int ic = min(i, p.seq - 1);              // rows past the end: a valid row's numbers, nothing of theirs is stored
+        const int ic = RAGGED ? min(i, p.seq - 1) : i; // rows past the end: a valid row's numbers, nothing of theirs is stored
         const long long sidx = ((long long)b * p.n_heads + h) * p.seq + ic;
         const float neg_lse2 = -p.lse[sidx] * LOG2E;
         float dlt;
@@ -641,7 +668,7 @@ attn_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                     float t8[8];
 #pragma unroll
                     for (int e = 0; e < 8; ++e) t8[e] = __uint_as_float(o[x + e]) * p.scale;
-                    if (i < p.seq) store8(row + c + x, t8);
+                    if (!RAGGED || i < p.seq) store8(row + c + x, t8);
                 }
             }
         }
@@ -701,7 +728,7 @@ __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gmem, u
 // 128 bytes and end inside its row: sequences that are a multiple of KV_BQ.  Otherwise the TMA warp loads them, one query per
 // lane, before it waits for the stage; queries past the end get lse = inf, so that their probabilities and dS are zero.  (A
 // flag at run time in place of the template cost the bulk form 1 % of the pass at 8 x 4096 tokens, head size 64.)
-template <int HD, bool STATS_BULK>
+template <int HD, bool RAGGED, bool STATS_BULK>
 __global__ void __launch_bounds__(KvDim<HD>::THREADS, KvDim<HD>::GROUPS == 1 ? 2 : 1)
 attn_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
                    const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const BwdParams p) {
@@ -775,28 +802,28 @@ attn_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 if (lane == 0) {
                     if (t == 0) {
                         mbar_arrive_expect_tx(kv_full, 2 * Q_BYTES);
-                        for (int c = 0; c < CH; ++c) tma_load_3d(k_smem + c * (BM * 128), &map_k, kv_full, kvh * p.k_col0_stride + c * 64, j0, b);
-                        for (int c = 0; c < CH; ++c) tma_load_3d(v_smem + c * (BM * 128), &map_v, kv_full, kvh * p.v_col0_stride + c * 64, j0, b);
+                        for (int c = 0; c < CH; ++c) load_box<RAGGED>(k_smem + c * (BM * 128), &map_k, kv_full, kvh * p.k_col0_stride + c * 64, j0, b, p.seq);
+                        for (int c = 0; c < CH; ++c) load_box<RAGGED>(v_smem + c * (BM * 128), &map_v, kv_full, kvh * p.v_col0_stride + c * 64, j0, b, p.seq);
                     }
                     mbar_arrive_expect_tx(&qdo_full[st], 2 * KV_Q_BYTES);
-                    for (int c = 0; c < CH; ++c) tma_load_3d(q_smem + st * KV_Q_BYTES + c * (KV_BQ * 128), &map_q, &qdo_full[st], h * p.q_col0_stride + c * 64, i0, b);
-                    for (int c = 0; c < CH; ++c) tma_load_3d(do_smem + st * KV_Q_BYTES + c * (KV_BQ * 128), &map_do, &qdo_full[st], h * p.do_col0_stride + c * 64, i0, b);
+                    for (int c = 0; c < CH; ++c) load_box<RAGGED>(q_smem + st * KV_Q_BYTES + c * (KV_BQ * 128), &map_q, &qdo_full[st], h * p.q_col0_stride + c * 64, i0, b, p.seq);
+                    for (int c = 0; c < CH; ++c) load_box<RAGGED>(do_smem + st * KV_Q_BYTES + c * (KV_BQ * 128), &map_do, &qdo_full[st], h * p.do_col0_stride + c * 64, i0, b, p.seq);
                 }
                 __syncwarp();
                 if (++st == KV_STAGES) { st = 0; sph ^= 1; }
             }
         } else if (lane == 0) {
             mbar_arrive_expect_tx(kv_full, 2 * Q_BYTES);
-            for (int c = 0; c < CH; ++c) tma_load_3d(k_smem + c * (BM * 128), &map_k, kv_full, kvh * p.k_col0_stride + c * 64, j0, b);
-            for (int c = 0; c < CH; ++c) tma_load_3d(v_smem + c * (BM * 128), &map_v, kv_full, kvh * p.v_col0_stride + c * 64, j0, b);
+            for (int c = 0; c < CH; ++c) load_box<RAGGED>(k_smem + c * (BM * 128), &map_k, kv_full, kvh * p.k_col0_stride + c * 64, j0, b, p.seq);
+            for (int c = 0; c < CH; ++c) load_box<RAGGED>(v_smem + c * (BM * 128), &map_v, kv_full, kvh * p.v_col0_stride + c * 64, j0, b, p.seq);
             int st = 0;
             uint32_t sph = 0;                           // stage of tile t and its phase parity (t / KV_STAGES) & 1
             for (int t = 0; t < n_tiles; ++t) {
                 const int i0 = (qs_lo + t) * KV_BQ;
                 if (!mbar_wait(&qdo_empty[st], sph ^ 1, abort_flag)) break;
                 mbar_arrive_expect_tx(&qdo_full[st], 2 * KV_Q_BYTES + KV_STATS_BYTES);
-                for (int c = 0; c < CH; ++c) tma_load_3d(q_smem + st * KV_Q_BYTES + c * (KV_BQ * 128), &map_q, &qdo_full[st], h * p.q_col0_stride + c * 64, i0, b);
-                for (int c = 0; c < CH; ++c) tma_load_3d(do_smem + st * KV_Q_BYTES + c * (KV_BQ * 128), &map_do, &qdo_full[st], h * p.do_col0_stride + c * 64, i0, b);
+                for (int c = 0; c < CH; ++c) load_box<RAGGED>(q_smem + st * KV_Q_BYTES + c * (KV_BQ * 128), &map_q, &qdo_full[st], h * p.q_col0_stride + c * 64, i0, b, p.seq);
+                for (int c = 0; c < CH; ++c) load_box<RAGGED>(do_smem + st * KV_Q_BYTES + c * (KV_BQ * 128), &map_do, &qdo_full[st], h * p.do_col0_stride + c * 64, i0, b, p.seq);
                 bulk_load_1d(stats + st * 2 * KV_BQ, p.lse + srow + i0, KV_BQ * 4, &qdo_full[st]);
                 bulk_load_1d(stats + st * 2 * KV_BQ + KV_BQ, p.delta + srow + i0, KV_BQ * 4, &qdo_full[st]);
                 if (++st == KV_STAGES) { st = 0; sph ^= 1; }
@@ -804,10 +831,11 @@ attn_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         }
     } else if (warp == 1 || warp == W_DP) {
         // ------------------------------------------------ MMA issuers 1 and 2: S^T = K Q^T (warp 1), dP^T = V dO^T (warp W_DP)
-        {
+        using I = Issue<HD != 256>;
+        if (I::joins(lane)) {
             constexpr uint32_t idesc_s = idesc_bf16_f32(BM, KV_BQ);
             const bool is_s = warp == 1;
-            bool ok = warp_wait(kv_full, 0, abort_flag);
+            bool ok = I::wait(kv_full, 0, abort_flag);
             const uint64_t ad = smem_desc_sw128(smem_u32(is_s ? k_smem : v_smem));
             int st = 0;
             uint32_t sph = 0;
@@ -815,54 +843,55 @@ attn_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 const int g = t & 1;
                 const uint32_t ph = (t >> 1) & 1;
                 // in place: the buffer also holds P^T / dS^T of tile t - 2 until that tile's dV / dK products are done
-                if (!warp_wait(&qdo_full[st], sph, abort_flag) || !warp_wait(INPLACE ? &pds_free[g] : &sdp_free[g], ph ^ 1, abort_flag)) { ok = false; break; }
+                if (!I::wait(&qdo_full[st], sph, abort_flag) || !I::wait(INPLACE ? &pds_free[g] : &sdp_free[g], ph ^ 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
-                if (elect_one()) {
-                const uint64_t bd = smem_desc_sw128(smem_u32((is_s ? q_smem : do_smem) + st * KV_Q_BYTES));
-                const uint32_t tmem_d = tmem_base + (is_s ? KV_S_COL : KV_DP_COL) + g * KV_BQ;
+                if (I::elected()) {
+                    const uint64_t bd = smem_desc_sw128(smem_u32((is_s ? q_smem : do_smem) + st * KV_Q_BYTES));
+                    const uint32_t tmem_d = tmem_base + (is_s ? KV_S_COL : KV_DP_COL) + g * KV_BQ;
 #pragma unroll
-                for (int c = 0; c < CH; ++c)
+                    for (int c = 0; c < CH; ++c)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        umma_bf16(tmem_d, ad + (uint64_t)(c * (BM * 128 / 16) + 2 * j), bd + (uint64_t)(c * (KV_BQ * 128 / 16) + 2 * j), idesc_s,
-                                  (c | j) != 0 ? 1u : 0u);
-                umma_commit(&sdp_full[g]);
+                        for (int j = 0; j < 4; ++j)
+                            umma_bf16(tmem_d, ad + (uint64_t)(c * (BM * 128 / 16) + 2 * j), bd + (uint64_t)(c * (KV_BQ * 128 / 16) + 2 * j), idesc_s,
+                                      (c | j) != 0 ? 1u : 0u);
+                    umma_commit(&sdp_full[g]);
                 }
-                __syncwarp();
+                I::done();
                 if (++st == KV_STAGES) { st = 0; sph ^= 1; }
             }
         }
     } else if (warp == W_ACC) {
         // ------------------------------------------------ MMA issuer 3: dV += P^T dO, dK += dS^T Q (this CTA's 128 columns)
-        {
+        using I = Issue<HD != 256>;
+        if (I::joins(lane)) {
             constexpr uint32_t idesc_acc = idesc_bf16_f32(BM, ACC) | IDESC_B_MN;
             bool ok = true;
             int st = 0;
             for (int t = 0; t < n_tiles && ok; ++t) {
                 const int g = t & 1;
                 const uint32_t ph = (t >> 1) & 1;
-                if (!warp_wait(&pds_full[g], ph, abort_flag)) { ok = false; break; }
+                if (!I::wait(&pds_full[g], ph, abort_flag)) { ok = false; break; }
                 tc_fence_after();
-                if (elect_one()) {
-                // A operands P^T / dS^T come from tensor memory (8 columns per 16 queries), B operands dO / Q MN-major from the stage
-                // separate: P^T at pa + {0, 8}, dS^T at pa + 16 + {0, 8}.  In place: P^T in the S^T buffer at +{0, 16}
-                // (the first 8 columns of each half's 16), dS^T in the dP^T buffer likewise
-                const uint32_t pa = tmem_base + (INPLACE ? KV_S_COL + g * KV_BQ : KV_PDS_COL + g * 32);
-                const uint32_t da = INPLACE ? tmem_base + KV_DP_COL + g * KV_BQ : pa + 16;
-                constexpr int A_STEP = INPLACE ? 16 : 8;
-                const uint64_t dod = smem_desc_mn_sw128(smem_u32(do_smem + st * KV_Q_BYTES + hh * (ACC / 64) * (KV_BQ * 128)), KV_BQ * 128);
-                const uint64_t qd = smem_desc_mn_sw128(smem_u32(q_smem + st * KV_Q_BYTES + hh * (ACC / 64) * (KV_BQ * 128)), KV_BQ * 128);
+                if (I::elected()) {
+                    // A operands P^T / dS^T come from tensor memory (8 columns per 16 queries), B operands dO / Q MN-major from the stage
+                    // separate: P^T at pa + {0, 8}, dS^T at pa + 16 + {0, 8}.  In place: P^T in the S^T buffer at +{0, 16}
+                    // (the first 8 columns of each half's 16), dS^T in the dP^T buffer likewise
+                    const uint32_t pa = tmem_base + (INPLACE ? KV_S_COL + g * KV_BQ : KV_PDS_COL + g * 32);
+                    const uint32_t da = INPLACE ? tmem_base + KV_DP_COL + g * KV_BQ : pa + 16;
+                    constexpr int A_STEP = INPLACE ? 16 : 8;
+                    const uint64_t dod = smem_desc_mn_sw128(smem_u32(do_smem + st * KV_Q_BYTES + hh * (ACC / 64) * (KV_BQ * 128)), KV_BQ * 128);
+                    const uint64_t qd = smem_desc_mn_sw128(smem_u32(q_smem + st * KV_Q_BYTES + hh * (ACC / 64) * (KV_BQ * 128)), KV_BQ * 128);
 #pragma unroll
-                for (int j = 0; j < 2; ++j)
-                    umma_bf16_ts(tmem_base + KV_DV_COL, pa + A_STEP * j, dod + (uint64_t)(j * (2048 / 16)), idesc_acc, (t | j) != 0 ? 1u : 0u);
+                    for (int j = 0; j < 2; ++j)
+                        umma_bf16_ts(tmem_base + KV_DV_COL, pa + A_STEP * j, dod + (uint64_t)(j * (2048 / 16)), idesc_acc, (t | j) != 0 ? 1u : 0u);
 #pragma unroll
-                for (int j = 0; j < 2; ++j)
-                    umma_bf16_ts(tmem_base + KV_DK_COL, da + A_STEP * j, qd + (uint64_t)(j * (2048 / 16)), idesc_acc, (t | j) != 0 ? 1u : 0u);
-                umma_commit(&qdo_empty[st]);
-                umma_commit(&pds_free[g]);
-                if (t == n_tiles - 1) umma_commit(acc_done);
+                    for (int j = 0; j < 2; ++j)
+                        umma_bf16_ts(tmem_base + KV_DK_COL, da + A_STEP * j, qd + (uint64_t)(j * (2048 / 16)), idesc_acc, (t | j) != 0 ? 1u : 0u);
+                    umma_commit(&qdo_empty[st]);
+                    umma_commit(&pds_free[g]);
+                    if (t == n_tiles - 1) umma_commit(acc_done);
                 }
-                __syncwarp();
+                I::done();
                 if (++st == KV_STAGES) st = 0;
             }
         }
@@ -938,13 +967,13 @@ attn_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 tmem_ld_32x32(lane_addr + KV_DK_COL + half * (ACC / 2) + c, o);
                 tmem_ld_wait();
 #pragma unroll
-                for (int x = 0; x < 32 && j < p.seq; x += 4)
+                for (int x = 0; x < 32 && (!RAGGED || j < p.seq); x += 4)
                     atomicAdd(reinterpret_cast<float4*>(krow + c + x), make_float4(__uint_as_float(o[x]) * p.scale, __uint_as_float(o[x + 1]) * p.scale,
                                                                                  __uint_as_float(o[x + 2]) * p.scale, __uint_as_float(o[x + 3]) * p.scale));
                 tmem_ld_32x32(lane_addr + KV_DV_COL + half * (ACC / 2) + c, o);
                 tmem_ld_wait();
 #pragma unroll
-                for (int x = 0; x < 32 && j < p.seq; x += 4)
+                for (int x = 0; x < 32 && (!RAGGED || j < p.seq); x += 4)
                     atomicAdd(reinterpret_cast<float4*>(vrow + c + x), make_float4(__uint_as_float(o[x]), __uint_as_float(o[x + 1]),
                                                                                  __uint_as_float(o[x + 2]), __uint_as_float(o[x + 3])));
             }
@@ -978,37 +1007,44 @@ int32_t launch_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorM
     MFT_LAUNCH_CHECK("attn_fwd_tc");
     return MFT_OK;
 }
-template <int HD>
-int32_t launch_dq(const CUtensorMap& mq, const CUtensorMap& md, const CUtensorMap& mk, const CUtensorMap& mv, const BwdParams& p, dim3 grid, cudaStream_t stream) {
+template <int HD, bool RAGGED>
+int32_t launch_dq_as(const CUtensorMap& mq, const CUtensorMap& md, const CUtensorMap& mk, const CUtensorMap& mv, const BwdParams& p, dim3 grid, cudaStream_t stream) {
     static PerDeviceFlag configured_on;           // function attributes are per device
     bool& configured = configured_on.here();
     if (!configured) {
-        if (int32_t s = check_cuda(cudaFuncSetAttribute(attn_dq_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, DqDim<HD>::SMEM), "attention smem attribute")) return s;
+        if (int32_t s = check_cuda(cudaFuncSetAttribute(attn_dq_tc_kernel<HD, RAGGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, DqDim<HD>::SMEM), "attention smem attribute")) return s;
         configured = true;
     }
-    launch_dep(attn_dq_tc_kernel<HD>, dim3(grid), dim3(DqDim<HD>::THREADS), (size_t)(DqDim<HD>::SMEM), stream, mq, md, mk, mv, p);
+    launch_dep(attn_dq_tc_kernel<HD, RAGGED>, dim3(grid), dim3(DqDim<HD>::THREADS), (size_t)(DqDim<HD>::SMEM), stream, mq, md, mk, mv, p);
     MFT_LAUNCH_CHECK("attn_dq_tc");
     return MFT_OK;
 }
-template <int HD, bool STATS_BULK>
+// Sequences of whole tiles keep the maps without a batch dimension: with the others, and no other change, the whole backward
+// pass took 252 instead of 211 us at 1 x 3072 tokens, 107 / 96 at 4 x 768 and 1774 / 1730 at 8 x 4096 (14 / 2 heads of 64).
+template <int HD>
+int32_t launch_dq(const CUtensorMap& mq, const CUtensorMap& md, const CUtensorMap& mk, const CUtensorMap& mv, const BwdParams& p, dim3 grid, cudaStream_t stream) {
+    return p.seq % BM ? launch_dq_as<HD, true>(mq, md, mk, mv, p, grid, stream) : launch_dq_as<HD, false>(mq, md, mk, mv, p, grid, stream);
+}
+template <int HD, bool RAGGED, bool STATS_BULK>
 int32_t launch_dkv_as(const CUtensorMap& mq, const CUtensorMap& md, const CUtensorMap& mk, const CUtensorMap& mv, const BwdParams& p, int seq, int n_heads, int batch,
                    cudaStream_t stream) {
     static PerDeviceFlag configured_on;           // function attributes are per device
     bool& configured = configured_on.here();
     if (!configured) {
-        if (int32_t s = check_cuda(cudaFuncSetAttribute(attn_dkv_tc_kernel<HD, STATS_BULK>, cudaFuncAttributeMaxDynamicSharedMemorySize, KvDim<HD>::SMEM), "attention smem attribute")) return s;
+        if (int32_t s = check_cuda(cudaFuncSetAttribute(attn_dkv_tc_kernel<HD, RAGGED, STATS_BULK>, cudaFuncAttributeMaxDynamicSharedMemorySize, KvDim<HD>::SMEM), "attention smem attribute")) return s;
         configured = true;
     }
     dim3 grid((unsigned)((seq + BM - 1) / BM), (unsigned)(KvDim<HD>::NPART * n_heads), (unsigned)batch);
-    launch_dep(attn_dkv_tc_kernel<HD, STATS_BULK>, dim3(grid), dim3(KvDim<HD>::THREADS), (size_t)(KvDim<HD>::SMEM), stream, mq, md, mk, mv, p);
+    launch_dep(attn_dkv_tc_kernel<HD, RAGGED, STATS_BULK>, dim3(grid), dim3(KvDim<HD>::THREADS), (size_t)(KvDim<HD>::SMEM), stream, mq, md, mk, mv, p);
     MFT_LAUNCH_CHECK("attn_dkv_tc");
     return MFT_OK;
 }
 template <int HD>
 int32_t launch_dkv(const CUtensorMap& mq, const CUtensorMap& md, const CUtensorMap& mk, const CUtensorMap& mv, const BwdParams& p, int seq, int n_heads, int batch,
                    cudaStream_t stream) {
-    return seq % KV_BQ == 0 ? launch_dkv_as<HD, true>(mq, md, mk, mv, p, seq, n_heads, batch, stream)
-                            : launch_dkv_as<HD, false>(mq, md, mk, mv, p, seq, n_heads, batch, stream);
+    return seq % BM == 0      ? launch_dkv_as<HD, false, true>(mq, md, mk, mv, p, seq, n_heads, batch, stream)
+           : seq % KV_BQ == 0 ? launch_dkv_as<HD, true, true>(mq, md, mk, mv, p, seq, n_heads, batch, stream)
+                              : launch_dkv_as<HD, true, false>(mq, md, mk, mv, p, seq, n_heads, batch, stream);
 }
 
 // Where the backward kernels win over the mma.sync pair.  Microseconds mma.sync / tcgen05 of the whole backward pass, batch
@@ -1050,6 +1086,12 @@ int32_t attn_fwd_sm100(const AttnParams& a, int hd, cudaStream_t stream) {
     return HD_DISPATCH(hd, launch_fwd<64>(mq, mk, mv, p, grid, stream), launch_fwd<128>(mq, mk, mv, p, grid, stream), launch_fwd<256>(mq, mk, mv, p, grid, stream));
 }
 
+// the tensor map that load_box<a.seq % BM != 0> reads through
+static int32_t box_map(CUtensorMap* map, const void* base, const AttnParams& a, int64_t cols, int64_t ld, int box_rows) {
+    return a.seq % BM ? make_tmap_bf16_batched(map, base, a.batch, a.seq, cols, ld, box_rows)
+                      : make_tmap_bf16(map, base, (int64_t)a.batch * a.seq, cols, ld, box_rows);
+}
+
 int32_t attn_dq_sm100(const AttnParams& a, int hd, bool compute_delta, cudaStream_t stream) {
     static const int enabled = [] { const char* e = std::getenv("MFT_ATTN_TC"); return e ? std::atoi(e) : 1; }();
     if (!enabled || !tc_shape_ok(hd) || !device_status_word()) return MFT_ERR_UNSUPPORTED;
@@ -1060,10 +1102,10 @@ int32_t attn_dq_sm100(const AttnParams& a, int hd, bool compute_delta, cudaStrea
     if (a.sq.stride_h % 8 || a.sk.stride_h % 8 || a.sv.stride_h % 8 || a.sdo.stride_h % 8) return MFT_ERR_UNSUPPORTED;
     if ((int64_t)a.batch * a.seq >= (1ll << 31)) return MFT_ERR_UNSUPPORTED;
     CUtensorMap mq, md, mk, mv;
-    if (make_tmap_bf16_batched(&mq, a.q, a.batch, a.seq, (int64_t)(a.n_heads - 1) * a.sq.stride_h + hd, a.sq.stride_s, BM) != MFT_OK) return MFT_ERR_UNSUPPORTED;
-    if (make_tmap_bf16_batched(&md, a.d_o, a.batch, a.seq, (int64_t)(a.n_heads - 1) * a.sdo.stride_h + hd, a.sdo.stride_s, BM) != MFT_OK) return MFT_ERR_UNSUPPORTED;
-    if (make_tmap_bf16_batched(&mk, a.k, a.batch, a.seq, (int64_t)(a.n_kv - 1) * a.sk.stride_h + hd, a.sk.stride_s, DQ_BN) != MFT_OK) return MFT_ERR_UNSUPPORTED;
-    if (make_tmap_bf16_batched(&mv, a.v, a.batch, a.seq, (int64_t)(a.n_kv - 1) * a.sv.stride_h + hd, a.sv.stride_s, DQ_BN) != MFT_OK) return MFT_ERR_UNSUPPORTED;
+    if (box_map(&mq, a.q, a, (int64_t)(a.n_heads - 1) * a.sq.stride_h + hd, a.sq.stride_s, BM) != MFT_OK) return MFT_ERR_UNSUPPORTED;
+    if (box_map(&md, a.d_o, a, (int64_t)(a.n_heads - 1) * a.sdo.stride_h + hd, a.sdo.stride_s, BM) != MFT_OK) return MFT_ERR_UNSUPPORTED;
+    if (box_map(&mk, a.k, a, (int64_t)(a.n_kv - 1) * a.sk.stride_h + hd, a.sk.stride_s, DQ_BN) != MFT_OK) return MFT_ERR_UNSUPPORTED;
+    if (box_map(&mv, a.v, a, (int64_t)(a.n_kv - 1) * a.sv.stride_h + hd, a.sv.stride_s, DQ_BN) != MFT_OK) return MFT_ERR_UNSUPPORTED;
     BwdParams p{};
     p.seq = a.seq; p.n_heads = a.n_heads; p.n_kv = a.n_kv; p.rep = a.rep; p.window = a.window; p.scale = a.scale;
     p.lse = a.lse; p.delta = a.delta; p.dq = a.dq; p.sq_b = a.sq.stride_b; p.sq_s = a.sq.stride_s; p.sq_h = a.sq.stride_h;
@@ -1089,10 +1131,10 @@ int32_t attn_dkv_sm100(const AttnParams& a, int hd, cudaStream_t stream) {
     if ((int64_t)a.batch * a.seq >= (1ll << 31) || 2 * a.n_heads > 65535) return MFT_ERR_UNSUPPORTED;
     if (!aligned16(a.lse) || !aligned16(a.delta) || !aligned16(a.dkv_acc)) return MFT_ERR_UNSUPPORTED;
     CUtensorMap mq, md, mk, mv;
-    if (make_tmap_bf16_batched(&mq, a.q, a.batch, a.seq, (int64_t)(a.n_heads - 1) * a.sq.stride_h + hd, a.sq.stride_s, KV_BQ) != MFT_OK) return MFT_ERR_UNSUPPORTED;
-    if (make_tmap_bf16_batched(&md, a.d_o, a.batch, a.seq, (int64_t)(a.n_heads - 1) * a.sdo.stride_h + hd, a.sdo.stride_s, KV_BQ) != MFT_OK) return MFT_ERR_UNSUPPORTED;
-    if (make_tmap_bf16_batched(&mk, a.k, a.batch, a.seq, (int64_t)(a.n_kv - 1) * a.sk.stride_h + hd, a.sk.stride_s, BM) != MFT_OK) return MFT_ERR_UNSUPPORTED;
-    if (make_tmap_bf16_batched(&mv, a.v, a.batch, a.seq, (int64_t)(a.n_kv - 1) * a.sv.stride_h + hd, a.sv.stride_s, BM) != MFT_OK) return MFT_ERR_UNSUPPORTED;
+    if (box_map(&mq, a.q, a, (int64_t)(a.n_heads - 1) * a.sq.stride_h + hd, a.sq.stride_s, KV_BQ) != MFT_OK) return MFT_ERR_UNSUPPORTED;
+    if (box_map(&md, a.d_o, a, (int64_t)(a.n_heads - 1) * a.sdo.stride_h + hd, a.sdo.stride_s, KV_BQ) != MFT_OK) return MFT_ERR_UNSUPPORTED;
+    if (box_map(&mk, a.k, a, (int64_t)(a.n_kv - 1) * a.sk.stride_h + hd, a.sk.stride_s, BM) != MFT_OK) return MFT_ERR_UNSUPPORTED;
+    if (box_map(&mv, a.v, a, (int64_t)(a.n_kv - 1) * a.sv.stride_h + hd, a.sv.stride_s, BM) != MFT_OK) return MFT_ERR_UNSUPPORTED;
     BwdParams p{};
     p.seq = a.seq; p.n_heads = a.n_heads; p.n_kv = a.n_kv; p.rep = a.rep; p.window = a.window; p.scale = a.scale;
     p.lse = a.lse; p.delta = a.delta; p.dq = a.dq; p.sq_b = a.sq.stride_b; p.sq_s = a.sq.stride_s; p.sq_h = a.sq.stride_h;
