@@ -1,10 +1,11 @@
 // RMSNorm / LayerNorm forward and backward, and the fused per-head
 // RMSNorm + rotary embedding used on Q and K.  Model-width RMSNorm rows up to
-// 2048 elements are handled one WARP per row (all of the row's 128-bit loads
-// in flight at once, shuffle reductions, no block barrier); wider rows and
-// LayerNorm use one CTA per row.  The row stays in registers between the
-// reduction and the write.  One warp per (token, head) for the per-head
-// kernel.  HBM-bound: every element is read once and written once.
+// 2048 elements are handled by a CTA of one to eight warps per row (one
+// 128-bit vector of every input per thread, all loads before the first sum),
+// forward calls of many rows by one warp per row; wider rows and LayerNorm use
+// one CTA per row.  The row stays in registers between the reduction and the
+// write.  One warp per (token, head) for the per-head kernel.  HBM-bound:
+// every element is read once and written once.
 #include <cmath>
 #include <vector>
 
@@ -193,6 +194,74 @@ rmsnorm_fwd_row_kernel(const TX* __restrict__ x, const float* __restrict__ w, fl
     }
 }
 
+// ---- one warp per row, for forward calls of many rows (VPL = 8-vectors a lane: (dim + 255) / 256)
+// A forward pass reads and writes so little per row that above a few thousand rows the row kernels are bound by starting and
+// ending their CTAs.  Four rows a CTA and no barrier there; below, the row kernels' shorter chain wins.  Same bits: vector k of
+// a lane is the vector of the row kernels' thread 32 k + lane, and the sums run in their order.
+// Microseconds row kernel / warp kernel, inputs in L2 where they fit.  Single norm, f32 -> bf16:  1600 x 640 2.94 / 3.07,
+// 2048 x 512 2.94 / 3.07,  2048 x 640 3.58 / 3.33,  3003 x 320 3.33 / 3.07,  4096 x 896 6.14 / 5.12,  8192 x 640 9.73 / 6.78,
+// 16384 x 640 18.1 / 11.1,  16384 x 1152 26.0 / 21.5.  Rows of more than 1536 columns leave five CTAs on an SM: 2960 rows fill
+// the chip once, and a second wave that is nearly empty loses (2400 x 2048 7.4 / 6.9,  4096 x 2048 10.9 / 12.2,  8192 22.0 / 20.4).
+// The fused pair:  3003 x 1152 9.6 / 9.7,  4096 x 1152 12.0 / 13.4,  6000 x 640 10.5 / 10.9,  8192 x 1152 24.2 / 23.0,
+// 16384 x 1152 45.7 / 42.1.  With a residual the row kernel is ahead everywhere (16384 x 1152 36.6 / 41.2).
+constexpr int WARP_ROWS = 4;      // rows per CTA
+inline dim3 warp_grid(int64_t rows) { return dim3((unsigned)((rows + WARP_ROWS - 1) / WARP_ROWS)); }
+inline bool warp_per_row_fwd(int64_t rows, int64_t dim) {
+    if (dim > ROW_MAX_DIM || dim <= 256) return false;
+    if (dim > 1536) return (rows >= 2048 && rows <= 2688) || rows >= 6000;
+    return rows >= (dim > 512 ? 2048 : 3000);
+}
+inline bool warp_per_row_add_norm(int64_t rows) { return rows >= 8192; }
+
+template <int VPL>
+__device__ __forceinline__ float warp_row_sum(const float (&v)[VPL][8]) {
+    float part[VPL], s = 0.f;
+#pragma unroll
+    for (int k = 0; k < VPL; ++k) {
+        part[k] = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) part[k] += v[k][j] * v[k][j];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < VPL; ++k) part[k] += __shfl_xor_sync(0xffffffffu, part[k], o);
+#pragma unroll
+    for (int k = 0; k < VPL; ++k) s += part[k];
+    return s;
+}
+
+template <typename TX, typename TY, int VPL>
+__global__ void __launch_bounds__(WARP_ROWS * 32)
+rmsnorm_fwd_warp_kernel(const TX* __restrict__ x, const float* __restrict__ w, float eps, int unit_offset,
+                        TY* __restrict__ y, float* __restrict__ rstd_out, int64_t rows, int64_t dim) {
+    dep_trigger();
+    dep_wait();
+    const int lane = threadIdx.x & 31, nvec = (int)(dim / 8);
+    const int64_t row = (int64_t)blockIdx.x * WARP_ROWS + (threadIdx.x >> 5);
+    if (row >= rows) return;
+    float v[VPL][8];
+#pragma unroll
+    for (int k = 0; k < VPL; ++k) {
+        const int i = lane + k * 32;
+        zero8(v[k]);
+        if (i < nvec) load8(x + row * dim + i * 8, v[k]);
+    }
+    const float rstd = rsqrtf(warp_row_sum<VPL>(v) / (float)dim + eps);
+    if (lane == 0 && rstd_out) rstd_out[row] = rstd;
+#pragma unroll
+    for (int k = 0; k < VPL; ++k) {
+        const int i = lane + k * 32;
+        if (i < nvec) {
+            float wv[8], o[8];
+            load8(w + i * 8, wv);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] = norm_out(v[k][j], rstd, unit_offset ? 1.0f + wv[j] : wv[j]);
+            store8(y + row * dim + i * 8, o);
+        }
+    }
+}
+
 template <typename TDY, typename TX, typename TDX>
 __global__ void __launch_bounds__(ROW_MAX_WARPS * 32)
 rmsnorm_bwd_row_kernel(const TDY* __restrict__ dy, const TX* __restrict__ x, const float* __restrict__ w,
@@ -279,6 +348,60 @@ rmsnorm_add_norm_fwd_kernel(const __nv_bfloat16* __restrict__ y, const float* __
 #pragma unroll
     for (int j = 0; j < 8; ++j) o[j] = norm_out(v[j], rn, unit_next ? 1.0f + wn[j] : wn[j]);
     store8(h_next + at, o);
+}
+
+// The same by one warp per row (see rmsnorm_fwd_warp_kernel)
+template <int VPL>
+__global__ void __launch_bounds__(WARP_ROWS * 32)
+rmsnorm_add_norm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ y, const float* __restrict__ w_post, int unit_post,
+                                 const float* __restrict__ residual, const float* __restrict__ w_next, int unit_next, float eps,
+                                 float* __restrict__ sum_out, float* __restrict__ rstd_post, __nv_bfloat16* __restrict__ h_next,
+                                 float* __restrict__ rstd_next, int64_t rows, int64_t dim) {
+    dep_trigger();
+    dep_wait();
+    const int lane = threadIdx.x & 31, nvec = (int)(dim / 8);
+    const int64_t row = (int64_t)blockIdx.x * WARP_ROWS + (threadIdx.x >> 5);
+    if (row >= rows) return;
+    float v[VPL][8];
+#pragma unroll
+    for (int k = 0; k < VPL; ++k) {
+        const int i = lane + k * 32;
+        zero8(v[k]);
+        if (i < nvec) load8(y + row * dim + i * 8, v[k]);
+    }
+    // the residual is read after the first sum: ask for its 32 bytes now, without holding registers for them
+#pragma unroll
+    for (int k = 0; k < VPL; ++k) {
+        const int i = lane + k * 32;
+        if (i < nvec) asm volatile("prefetch.global.L1 [%0];" ::"l"(residual + row * dim + i * 8));
+    }
+    const float rp = rsqrtf(warp_row_sum<VPL>(v) / (float)dim + eps);
+    if (lane == 0) rstd_post[row] = rp;
+#pragma unroll
+    for (int k = 0; k < VPL; ++k) {
+        const int i = lane + k * 32;
+        if (i < nvec) {
+            float wv[8], r[8];
+            load8(w_post + i * 8, wv);
+            load8(residual + row * dim + i * 8, r);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[k][j] = __fadd_rn(r[j], norm_out(v[k][j], rp, unit_post ? 1.0f + wv[j] : wv[j]));
+            store8(sum_out + row * dim + i * 8, v[k]);
+        }
+    }
+    const float rn = rsqrtf(warp_row_sum<VPL>(v) / (float)dim + eps);
+    if (lane == 0) rstd_next[row] = rn;
+#pragma unroll
+    for (int k = 0; k < VPL; ++k) {
+        const int i = lane + k * 32;
+        if (i < nvec) {
+            float wv[8], o[8];
+            load8(w_next + i * 8, wv);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] = norm_out(v[k][j], rn, unit_next ? 1.0f + wv[j] : wv[j]);
+            store8(h_next + row * dim + i * 8, o);
+        }
+    }
 }
 
 // Backward of the same pair: dx (f32, the gradient on x_sum that came down the residual path) first receives the
@@ -655,11 +778,14 @@ int32_t mft_rmsnorm_fwd(const void* x, int32_t xd, const float* w, float eps, in
     MFT_CHECK_ARG(y || (residual && sum_out), "mft_rmsnorm_fwd: nothing to write");
     MFT_CHECK_ARG(!residual || sum_out, "mft_rmsnorm_fwd: residual needs sum_out");
     MFT_CHECK_ARG(dim % 8 == 0 && dim <= 8 * NORM_THREADS * NORM_VPT, "mft_rmsnorm_fwd: dim must be a multiple of 8 and <= 4096");
+#define WARP(TX, TY, VPL) case VPL: launch_dep(rmsnorm_fwd_warp_kernel<TX, TY, VPL>, warp_grid(rows), dim3(WARP_ROWS * 32), (size_t)(0), as_stream(stream), (const TX*)x, w, eps, unit_offset, (TY*)y, rstd, rows, dim); break;
 #define CALL(TX, TY)                                                                                     \
-    if (dim <= ROW_MAX_DIM) launch_dep(rmsnorm_fwd_row_kernel<TX, TY>, row_grid(rows, dim), row_block(dim), (size_t)(0), as_stream(stream), (const TX*)x, w, eps, unit_offset, (TY*)y, rstd, residual, sum_out, rows, dim); \
+    if (!residual && warp_per_row_fwd(rows, dim)) switch ((dim + 255) / 256) { WARP(TX, TY, 2) WARP(TX, TY, 3) WARP(TX, TY, 4) WARP(TX, TY, 5) WARP(TX, TY, 6) WARP(TX, TY, 7) WARP(TX, TY, 8) } \
+    else if (dim <= ROW_MAX_DIM) launch_dep(rmsnorm_fwd_row_kernel<TX, TY>, row_grid(rows, dim), row_block(dim), (size_t)(0), as_stream(stream), (const TX*)x, w, eps, unit_offset, (TY*)y, rstd, residual, sum_out, rows, dim); \
     else launch_dep(rmsnorm_fwd_kernel<TX, TY>, dim3((unsigned)rows), dim3(NORM_THREADS), (size_t)(0), as_stream(stream), (const TX*)x, w, eps, unit_offset, (TY*)y, rstd, residual, sum_out, dim);
     DISPATCH_2(xd, yd, CALL)
 #undef CALL
+#undef WARP
     MFT_LAUNCH_CHECK("rmsnorm_fwd");
     return MFT_OK;
 }
@@ -688,9 +814,15 @@ int32_t mft_rmsnorm_add_norm_fwd(const void* y_bf16, const float* w_post, int32_
     MFT_CHECK_ARG(y_bf16 && w_post && residual && w_next && sum_out && rstd_post && h_next_bf16 && rstd_next && rows > 0, "mft_rmsnorm_add_norm_fwd: bad argument");
     MFT_CHECK_ARG(dim > 0 && dim % 8 == 0, "mft_rmsnorm_add_norm_fwd: dim must be a multiple of 8");
     if (dim > ROW_MAX_DIM) return fail(MFT_ERR_UNSUPPORTED, "mft_rmsnorm_add_norm_fwd: rows wider than 2048 use the separate norm calls");
-    launch_dep(rmsnorm_add_norm_fwd_kernel, row_grid(rows, dim), row_block(dim), (size_t)0, as_stream(stream),
-               (const __nv_bfloat16*)y_bf16, w_post, (int)unit_post, residual, w_next, (int)unit_next, eps, sum_out, rstd_post,
-               (__nv_bfloat16*)h_next_bf16, rstd_next, rows, dim);
+#define WARP(VPL) case VPL: launch_dep(rmsnorm_add_norm_fwd_warp_kernel<VPL>, warp_grid(rows), dim3(WARP_ROWS * 32), (size_t)0, as_stream(stream), \
+                                       (const __nv_bfloat16*)y_bf16, w_post, (int)unit_post, residual, w_next, (int)unit_next, eps, sum_out, rstd_post, \
+                                       (__nv_bfloat16*)h_next_bf16, rstd_next, rows, dim); break;
+    if (warp_per_row_add_norm(rows)) switch ((dim + 255) / 256) { WARP(1) WARP(2) WARP(3) WARP(4) WARP(5) WARP(6) WARP(7) WARP(8) }
+    else
+        launch_dep(rmsnorm_add_norm_fwd_kernel, row_grid(rows, dim), row_block(dim), (size_t)0, as_stream(stream),
+                   (const __nv_bfloat16*)y_bf16, w_post, (int)unit_post, residual, w_next, (int)unit_next, eps, sum_out, rstd_post,
+                   (__nv_bfloat16*)h_next_bf16, rstd_next, rows, dim);
+#undef WARP
     MFT_LAUNCH_CHECK("rmsnorm_add_norm_fwd");
     return MFT_OK;
 }
