@@ -11,11 +11,14 @@
 // memory in rank order, so the result does not depend on timing.  plan() below picks by the FMA time of the SM that gets
 // the most work.
 //
+// A product of at most one or two 32 x 32 tiles per SM under a short K goes to matmul_f32_small_kernel: see small_tiles().
+//
 // Measured: 4096^3 48.8 TFLOP/s, 512 x 4864 x 896 28.6 and 512 x 896 x 4864 27.5; one output per thread on 32 x 32 tiles
 // ran all of them at 5.2 (the f32 gated MLP of 512 tokens at 896 / 4864, forward and backward: 5.13 -> 0.96 ms).
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "gemm_sm100.h"
 
 namespace mft {
 namespace {
@@ -179,12 +182,35 @@ matmul_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, floa
     cluster.sync();       // nobody leaves while its partial tile is still being read
 }
 
+// One output per thread from 32 x 32 tiles: a small product is bound by the latency of its serial k loop, which 32 warps of
+// one FMA and two shared-memory reads a step walk faster than the two warps of a 64 x 64 tile.
+__global__ void __launch_bounds__(1024)
+matmul_f32_small_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C, int M, int N, int K, int64_t stride_a,
+                        int64_t stride_b, int64_t stride_c, int trans_b) {
+    __shared__ float as[32][33], bs[32][33];
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int row = blockIdx.y * 32 + ty, n0 = blockIdx.x * 32, col = n0 + tx;
+    const float* a = A + blockIdx.z * stride_a;
+    const float* b = B + blockIdx.z * stride_b;
+    float acc = 0.f;
+    for (int k0 = 0; k0 < K; k0 += 32) {
+        as[ty][tx] = (row < M && k0 + tx < K) ? a[(int64_t)row * K + k0 + tx] : 0.f;
+        if (trans_b) bs[tx][ty] = (k0 + tx < K && n0 + ty < N) ? b[(int64_t)(n0 + ty) * K + k0 + tx] : 0.f;      // rows of B side by side
+        else bs[ty][tx] = (k0 + ty < K && col < N) ? b[(int64_t)(k0 + ty) * N + col] : 0.f;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 32; ++k) acc = fmaf(as[ty][k], bs[k][tx], acc);
+        __syncthreads();
+    }
+    if (row < M && col < N) C[blockIdx.z * stride_c + (int64_t)row * N + col] = acc;
+}
+
 struct MmPlan { bool big; int splits; };
-// FMA time of the busiest SM in units of one 64 x 64 x 1 slab, tiles dealt round to the 148 SMs.  A 64 x 64 tile re-reads
+// FMA time of the busiest SM in units of one 64 x 64 x 1 slab, tiles dealt round to the SMs.  A 64 x 64 tile re-reads
 // its operands more often and has two warps to hide latency with: charged 15 %; each extra K range 64 steps for its pass
 // through shared memory.
 MmPlan plan(int64_t m, int64_t n, int64_t k, int64_t batch) {
-    const int64_t sms = 148;
+    const int64_t sms = num_sms();
     const int64_t big_tiles = ((m + 127) / 128) * ((n + 127) / 128) * batch, small_tiles = ((m + 63) / 64) * ((n + 63) / 64) * batch;
     MmPlan best{true, 1};
     double cost = (double)((big_tiles + sms - 1) / sms) * 4.0 * (double)k;
@@ -194,6 +220,17 @@ MmPlan plan(int64_t m, int64_t n, int64_t k, int64_t batch) {
         if (c < cost) { cost = c; best = {false, sp}; }
     }
     return best;
+}
+
+// Where the 32 x 32 tiles are the faster ones.  Microseconds 32 x 32 / register-blocked for one 128 x 128 product (16 tiles):
+//   B [K,N]:  K = 32 3.5 / 5.3,  128 8.1 / 13.3,  256 15 / 16.5,  384 21.6 / 22,  512 28 / 15.6 (cut over a cluster from there on)
+//   B [N,K]:  K = 32 3.8 / 5.1,  128 8.3 / 12.5,  192 12 / 17.4,  256 15 / 15.1
+// up to one tile per SM.  With two (256 products of 16 x 16), B [K,N] is even or ahead while K is not cut: K = 8 4.9 / 3.6,
+// 32 5.0 / 5.1,  64 8.2 / 8.4,  192 19.2 / 20.2,  1024 90.6 / 95.5;  B [N,K] behind: 8.7 / 7.7 at 64.
+bool small_tiles(int64_t m, int64_t n, int64_t k, int64_t batch, bool trans_b, const MmPlan& p) {
+    const int64_t tiles = ((m + 31) / 32) * ((n + 31) / 32) * batch, sms = num_sms();
+    if (tiles <= sms && k < (trans_b ? 256 : 448)) return true;
+    return !trans_b && tiles <= 2 * sms && !p.big && p.splits == 1 && k >= 32;
 }
 
 template <int BM, int BN, bool TRANS_B, bool VEC>
@@ -236,6 +273,12 @@ extern "C" int32_t mft_matmul_f32(const float* a, const float* b, float* c, int6
     MFT_CHECK_ARG(a && b && c && batch > 0 && m > 0 && n > 0 && k > 0 && batch <= 65535, "mft_matmul_f32: bad argument");
     MFT_CHECK_ARG(m < (1ll << 31) - 128 && n < (1ll << 31) - 128 && k < (1ll << 31) - 128, "mft_matmul_f32: dimension too large");
     const MmPlan p = plan(m, n, k, batch);
+    if (small_tiles(m, n, k, batch, trans_b != 0, p)) {
+        matmul_f32_small_kernel<<<dim3((unsigned)((n + 31) / 32), (unsigned)((m + 31) / 32), (unsigned)batch), dim3(32, 32), 0, as_stream(stream)>>>(
+            a, b, c, (int)m, (int)n, (int)k, stride_a, stride_b, stride_c, trans_b);
+        MFT_LAUNCH_CHECK("matmul_f32");
+        return MFT_OK;
+    }
     // 16-byte accesses need rows that start and end on 16 bytes in all three operands
     auto al = [](const void* q, int64_t stride) { return reinterpret_cast<uintptr_t>(q) % 16 == 0 && stride % 4 == 0; };
     const bool vec = k % 4 == 0 && n % 4 == 0 && al(a, stride_a) && al(b, stride_b) && al(c, stride_c);
