@@ -54,6 +54,8 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t a, uint32_
     asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
+__device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t v) { asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+
 // eight columns of one output row
 __device__ __forceinline__ void store_cols8(const GemmParams& p, int row, int col, float (&v)[8]) {
     if (row >= p.m || col >= p.n) return;
@@ -83,6 +85,7 @@ gemm_nt_ksplit_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     uint64_t* tmem_full_bar = bars + 2 * Cfg::STAGES;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_full_bar + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    volatile int* cluster_failed = abort_flag + 1;      // some CTA of the cluster gave up: set by that CTA in all of them
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int splits = p.splits, rank = (int)(blockIdx.x % splits), tile = (int)(blockIdx.x / splits);
@@ -94,6 +97,7 @@ gemm_nt_ksplit_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         for (int s = 0; s < Cfg::STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
         mbar_init(tmem_full_bar, 1);
         *abort_flag = 0;
+        *cluster_failed = 0;
         fence_barrier_init();
         tma_prefetch_desc(&map_a); tma_prefetch_desc(&map_b);
         if (p.k2 > 0) { tma_prefetch_desc(&map_a2); tma_prefetch_desc(&map_b2); }
@@ -107,8 +111,8 @@ gemm_nt_ksplit_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
 
     if (warp == 0) {
         if (lane == 0) {
-            int stage = 0; uint32_t phase = 0;
-            for (int kb = kb0; kb < kb1; ++kb) {
+            int stage = 0, issued = 0; uint32_t phase = 0;
+            for (int kb = kb0; kb < kb1; ++kb, ++issued) {
                 if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) break;
                 uint8_t* sa = tiles + stage * Cfg::STAGE_BYTES;
                 mbar_arrive_expect_tx(&full_bar[stage], Cfg::STAGE_BYTES);
@@ -118,6 +122,8 @@ gemm_nt_ksplit_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                 tma_load_2d(sa + Cfg::A_BYTES, main_kb ? &map_b : &map_b2, &full_bar[stage], k0, n0);
                 if (++stage == Cfg::STAGES) { stage = 0; phase ^= 1; }
             }
+            // the stages become the cluster's exchange area: no load of this CTA may land in them after a wait ran out
+            if (!mbar_wait(tmem_full_bar, 0, abort_flag)) drain_loads(full_bar, Cfg::STAGES, issued);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -159,6 +165,7 @@ gemm_nt_ksplit_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     const int groups_n = min(G, (p.n - n0 + 7) / 8);           // groups that exist
     // every MMA of the cluster has read its operands: the stages of all CTAs may be overwritten
     ks_cluster_sync();
+    if (threadIdx.x < splits && *abort_flag) st_cluster_u32(map_rank(smem_u32(const_cast<int*>(cluster_failed)), threadIdx.x), 1u);
     const int per_src = ((G + splits - 1) / splits) * 2 * Cfg::EX_ROWS;      // float4 per source rank
     if (epi && landed) {
         const uint32_t ex = smem_u32(tiles) + (uint32_t)((rank * per_src + row_in_tile) * 16);
@@ -184,7 +191,7 @@ gemm_nt_ksplit_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     }
     __syncwarp();
     ks_cluster_sync();
-    {
+    if (*cluster_failed == 0) {                 // (a rank that gave up sent nothing: the exchange area holds operand bytes in its place)
         const int g0 = rank * G / splits, ng = min((rank + 1) * G / splits, groups_n) - g0;
         const float4* ex = reinterpret_cast<const float4*>(tiles);
         // consecutive threads: consecutive groups of a row (contiguous bytes of D)

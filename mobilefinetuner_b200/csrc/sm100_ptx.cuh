@@ -76,6 +76,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     }
 }
 
+// For a CTA that gives up: bounded wait for its own loads that may still be in flight.  `issued` loads were armed round robin
+// on the `stages` barriers of `full`; the last one on a stage completes that barrier's phase number (times armed - 1).
+__device__ __forceinline__ void drain_loads(uint64_t* full, int stages, int issued) {
+    const unsigned long long t0 = globaltimer_ns();
+    for (int s = 0; s < stages && s < issued; ++s) {
+        const uint32_t last = (uint32_t)((issued - 1 - s) / stages);
+        while (!mbar_try_wait(&full[s], last & 1u) && globaltimer_ns() - t0 < WAIT_LIMIT_NS) {}
+    }
+}
+
 // ---- TMA (2-D tiled load into this CTA's shared memory)
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int32_t c0, int32_t c1) {
     asm volatile(
