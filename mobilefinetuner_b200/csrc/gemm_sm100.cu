@@ -92,7 +92,7 @@ gemm_nt_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (warp == 0) {
         // ------------------------------------------------ TMA producer
         if (lane == 0) {
-            int stage = 0; uint32_t phase = 0;
+            int stage = 0, issued = 0; uint32_t phase = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
                 const int t2 = tile % p.tiles_mn, split = tile / p.tiles_mn;
@@ -112,13 +112,10 @@ gemm_nt_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         tma_load_2d(sb, &map_b2, &full_bar[stage], 0, n0);
                     }
                     if (++stage == Cfg::STAGES) { stage = 0; phase ^= 1; }
+                    ++issued;
                 }
             }
-            if (!ok) {
-                // give loads still in flight a bounded chance to land before the CTA leaves
-                for (int s = 0; s < Cfg::STAGES; ++s)
-                    for (int i = 0; i < 4096 && !mbar_try_wait(&full_bar[s], 0) && !mbar_try_wait(&full_bar[s], 1); ++i) {}
-            }
+            if (!ok) drain_loads(full_bar, Cfg::STAGES, issued);     // nothing may land after the CTA has left
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer (warp-uniform loop, one elected lane issues: see the pair kernel)
