@@ -16,7 +16,7 @@
 //     512 x   32 x 13824   55.0 -> 12.9          4096 x  16 x 6912   30.2 -> 15.2
 #include <cuda.h>
 
-#include <cstdlib>
+#include <atomic>
 
 #include "common.cuh"
 #include "gemm_sm100.h"
@@ -249,36 +249,40 @@ int32_t launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& 
 
 }  // namespace
 
-// Clusters of S CTAs that run at the same time: the SMs of a GPC come in pairs that S has to fit into, so the count is
-// the driver's answer (B200: 74 of 2, 33 of 4, 15 of 8), asked once.
-static int active_clusters(int bn, int s) {
-    static int known[2][MAX_SPLIT + 1] = {};
-    int& n = known[bn == 128][s];
-    if (n == 0) {
-        n = num_sms() / s;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3((unsigned)(n * s));
-        cfg.blockDim = dim3(THREADS);
-        cfg.dynamicSmemBytes = bn == 128 ? KsCfg<128>::SMEM_BYTES : KsCfg<64>::SMEM_BYTES;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)s; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int got = 0;
-        cudaError_t e = bn == 128 ? cudaFuncSetAttribute(gemm_nt_ksplit_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, KsCfg<128>::SMEM_BYTES)
-                                  : cudaFuncSetAttribute(gemm_nt_ksplit_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, KsCfg<64>::SMEM_BYTES);
-        if (e == cudaSuccess)
-            e = bn == 128 ? cudaOccupancyMaxActiveClusters(&got, gemm_nt_ksplit_kernel<128>, &cfg) : cudaOccupancyMaxActiveClusters(&got, gemm_nt_ksplit_kernel<64>, &cfg);
-        if (e == cudaSuccess && got > 0) n = got;
-        else cudaGetLastError();
-    }
-    return n;
+// Clusters of S CTAs that run at the same time on this device: the SMs of a GPC come in pairs that S has to fit into, so the
+// count is the driver's answer (B200: 74 of 2, 33 of 4, 15 of 8), asked once per device.  0: the driver gives none or no answer,
+// and no plan has clusters of this size.  Threads that ask at the same time write the same value.
+static int active_clusters(int dev, int bn, int s) {
+    constexpr int NOT_ASKED = 0, NONE = -1, DEVICES = 64;
+    static std::atomic<int> known[DEVICES][2][MAX_SPLIT + 1] = {};
+    if (dev < 0 || dev >= DEVICES) return 0;
+    std::atomic<int>& entry = known[dev][bn == 128][s];
+    const int seen = entry.load(std::memory_order_relaxed);
+    if (seen != NOT_ASKED) return seen == NONE ? 0 : seen;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(num_sms() / s * s));
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = bn == 128 ? KsCfg<128>::SMEM_BYTES : KsCfg<64>::SMEM_BYTES;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)s; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int got = 0;
+    cudaError_t e = bn == 128 ? cudaFuncSetAttribute(gemm_nt_ksplit_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, KsCfg<128>::SMEM_BYTES)
+                              : cudaFuncSetAttribute(gemm_nt_ksplit_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, KsCfg<64>::SMEM_BYTES);
+    if (e == cudaSuccess)
+        e = bn == 128 ? cudaOccupancyMaxActiveClusters(&got, gemm_nt_ksplit_kernel<128>, &cfg) : cudaOccupancyMaxActiveClusters(&got, gemm_nt_ksplit_kernel<64>, &cfg);
+    if (e != cudaSuccess) { got = 0; cudaGetLastError(); }
+    entry.store(got > 0 ? got : NONE, std::memory_order_relaxed);
+    return got > 0 ? got : 0;
 }
 
 // Tile width (64 or 128; 0 = not this kernel) and K ranges for a bf16 plain-store call of this shape.  Times in ns.
 KsplitPlan ksplit_plan(int64_t m, int64_t n, int64_t k, int64_t k2) {
     KsplitPlan best;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return best; }
     const int64_t sms = num_sms(), kb = (k + BK - 1) / BK + (k2 > 0 ? 1 : 0);
     // what the persistent kernels take (measured on launches of one wave): 300 ns per k-block of a 256 x 256 pair tile,
     // 270 ns of a 128 x 64 single-CTA tile, plus the end of the last tile
@@ -295,7 +299,7 @@ KsplitPlan ksplit_plan(int64_t m, int64_t n, int64_t k, int64_t k2) {
         if (bn == 128 && n <= 64) continue;
         const int64_t tiles = ((m + BM - 1) / BM) * ((n + bn - 1) / bn);
         for (int sp = 2; sp <= MAX_SPLIT && kb / sp >= 4; ++sp) {      // (shorter ranges gain less than the exchange costs)
-            const int64_t clusters = active_clusters(bn, sp);
+            const int64_t clusters = active_clusters(dev, bn, sp);
             if (tiles > clusters) continue;             // one tile per CTA: a second wave repeats the start-up
             const double cost = (double)((kb + sp - 1) / sp) * (bn == 128 ? 300.0 : 270.0) + (bn == 128 ? 6500.0 : 5000.0);
             if (cost < best_cost) { best_cost = cost; best = {bn, sp}; }
