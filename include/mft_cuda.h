@@ -228,11 +228,16 @@ int32_t mft_gemm_nt(const void* a_bf16, int64_t lda, const void* b_bf16, int64_t
                     const float* bias, float alpha,
                     void* d, int64_t ldd, int32_t d_dtype, int32_t accumulate,
                     mft_stream_t stream);
-/* Tile plan of mft_gemm_nt for a plain call (no accumulate) of this shape: *tile_cols_host = columns of the CTA-pair
- * kernel's tile - 256, or 384 when the width is a multiple of 384, m a multiple of 256 and the cost model (waves of
- * tiles x k-blocks per tile) prefers the wider tile; f32 outputs take it only under at least 64 k-blocks per tile - or
- * 0 when another kernel takes the call.  Needs an initialised device (the SM count enters the plan). */
+/* Tile plan of the CTA-pair kernel for a plain mft_gemm_nt call (no accumulate) of this shape: *tile_cols_host = columns
+ * of its tile - 256, or 384 where n >= 384, m is a multiple of 256 and the cost model (waves of tiles x k-blocks per
+ * tile) prefers the wider tile; f32 outputs take it only under at least 64 k-blocks per tile - or 0 when the call is too
+ * small for that kernel (m < 256 or n < 192).  A bf16 output of few tiles does not get there: ask
+ * mft_gemm_nt_ksplit_plan first.  The SM count enters the plan (148 without a device). */
 int32_t mft_gemm_nt_tile_cols(int64_t m, int64_t n, int64_t k, int64_t k2, int32_t d_dtype, int32_t* tile_cols_host);
+/* Plan of the K-split kernel, which takes a plain mft_gemm_nt call with a bf16 output (16-byte aligned, ldd a multiple of
+ * 8) of this shape before the others: *tile_cols_host = columns of its tile (64 or 128) and *k_ranges_host = CTAs of the
+ * cluster that share a tile's K (2 .. 8), or 0 and 1 when another kernel is the faster one (always without a device). */
+int32_t mft_gemm_nt_ksplit_plan(int64_t m, int64_t n, int64_t k, int64_t k2, int32_t* tile_cols_host, int32_t* k_ranges_host);
 /* Measurement aid: bytes per clock that one SM takes in from L2 through its TMA unit when nothing else uses its shared
  * memory (one CTA per SM loads an L2-resident 64 MiB matrix into a ring of `stages` 32 KB stages that a second thread
  * releases at once).  mode 0: two tensor boxes of 128 rows x 128 bytes per stage (what the GEMMs load); 1: two bulk

@@ -485,10 +485,15 @@ int32_t gemm_nt_run(const GemmCall& c, cudaStream_t stream) {
     return s;
 }
 
+// The cluster kernels go first: K split over a cluster for bf16 outputs of few tiles, then CTA pairs (256 x 256 tiles).
+// MFT_GEMM_2CTA=0 selects the single-CTA kernel everywhere.
+static bool gemm_ksplit_enabled() {
+    static const int use_clusters = [] { const char* e = std::getenv("MFT_GEMM_2CTA"); return e ? std::atoi(e) : 1; }();
+    return use_clusters && device_status_word();
+}
+
 static int32_t gemm_nt_run_inner(const GemmCall& c, cudaStream_t stream) {
-    // CTA-pair kernel first (256 x 256 cluster tiles); MFT_GEMM_2CTA=0 selects the single-CTA kernel everywhere
-    static const int use_pair = [] { const char* e = std::getenv("MFT_GEMM_2CTA"); return e ? std::atoi(e) : 1; }();
-    if (use_pair && device_status_word()) {
+    if (gemm_ksplit_enabled()) {
         const int32_t s1 = gemm_nt_run_ksplit(c, stream);
         if (s1 != MFT_ERR_UNSUPPORTED) return s1;
         const int32_t s2 = gemm_nt_run_2cta(c, stream);
@@ -620,6 +625,14 @@ extern "C" int32_t mft_gemm_nt_tile_cols(int64_t m, int64_t n, int64_t k, int64_
     MFT_CHECK_ARG(tile_cols_host && m > 0 && n > 0 && k > 0 && k2 >= 0, "mft_gemm_nt_tile_cols: bad argument");
     MFT_CHECK_ARG(d_dtype == MFT_F32 || d_dtype == MFT_BF16, "mft_gemm_nt_tile_cols: D must be f32 or bf16");
     *tile_cols_host = gemm_nt_pair_tile_cols(m, n, k, k2, d_dtype == MFT_F32);
+    return MFT_OK;
+}
+
+extern "C" int32_t mft_gemm_nt_ksplit_plan(int64_t m, int64_t n, int64_t k, int64_t k2, int32_t* tile_cols_host, int32_t* k_ranges_host) {
+    MFT_CHECK_ARG(tile_cols_host && k_ranges_host && m > 0 && n > 0 && k > 0 && k2 >= 0, "mft_gemm_nt_ksplit_plan: bad argument");
+    const KsplitPlan plan = gemm_ksplit_enabled() ? ksplit_plan(m, n, k, k2) : KsplitPlan{};
+    *tile_cols_host = plan.bn;
+    *k_ranges_host = plan.splits;
     return MFT_OK;
 }
 

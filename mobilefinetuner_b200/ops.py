@@ -61,11 +61,20 @@ def gemm_nt(a, b, *, a2=None, b2=None, bias=None, alpha=1.0, out=None, out_dtype
 
 
 def gemm_nt_tile_cols(m, n, k, k2=0, out_dtype=BF16):
-    """Columns of the CTA-pair kernel's tile for a gemm_nt call of this shape (256 / 384), 0 when another kernel runs it."""
+    """Columns of the CTA-pair kernel's tile for a gemm_nt call of this shape (256 / 384), 0 when it is too small for that
+    kernel.  bf16 outputs of few tiles go to the K-split kernel before it: gemm_nt_ksplit_plan."""
     L.init(torch.cuda.current_device())
     cols = C.c_int32(0)
     L.call("mft_gemm_nt_tile_cols", m, n, k, k2, L.MFT_BF16 if out_dtype == BF16 else L.MFT_F32, C.byref(cols))
     return cols.value
+
+
+def gemm_nt_ksplit_plan(m, n, k, k2=0):
+    """(tile columns, K ranges) with which the K-split kernel takes a bf16 gemm_nt call of this shape, (0, 1) when it does not."""
+    L.init(torch.cuda.current_device())
+    cols, ranges = C.c_int32(0), C.c_int32(0)
+    L.call("mft_gemm_nt_ksplit_plan", m, n, k, k2, C.byref(cols), C.byref(ranges))
+    return cols.value, ranges.value
 
 
 def gemm_tn_acc(u, v, out, alpha=1.0):

@@ -6,20 +6,16 @@ pytestmark = pytest.mark.gpu
 BF = torch.bfloat16
 
 
-@pytest.mark.parametrize("m,n,k,k2,bias", [
-    (512, 16, 13824, 0, False), (512, 48, 1152, 0, False), (130, 40, 520, 0, False), (512, 1152, 13824, 32, False), (512, 1536, 1152, 48, False), (1, 64, 704, 0, False),
-    (129, 72, 1352, 16, True), (437, 640, 2048, 8, False), (437, 8, 640, 0, False), (512, 2304, 768, 8, True), (65, 128, 1000, 0, True),
-    (1985, 896, 4864, 0, False), (300, 200, 1160, 64, True), (512, 50, 6912, 0, True), (1000, 768, 3072, 0, False)])
-def test_gemm_ksplit(m, n, k, k2, bias):
+def _check(m, n, k, k2, bias):
     from mobilefinetuner_b200 import ops as O
     g = torch.Generator(device="cuda").manual_seed(m * 131 + n * 7 + k)
 
     def rnd(r, c, scale=1.0):
         return (torch.randn(r, c, device="cuda", generator=g) * scale).to(BF)
     a, b = rnd(m, k), rnd(n, k, 0.05)
-    a2, b2 = (rnd(m, 64)[:, :k2], rnd(n, 64, 0.05)[:, :k2]) if k2 else (None, None)
-    if k2 % 16:      # the second segment's columns up to the next multiple of 16 take part: zero, as the rank panels are
-        a2, b2 = torch.zeros(m, 64, device="cuda", dtype=BF), torch.zeros(n, 64, device="cuda", dtype=BF)
+    a2 = b2 = None
+    if k2:           # panels of 64 columns: what lies past the second segment must not be read
+        a2, b2 = torch.full((m, 64), float("nan"), device="cuda", dtype=BF), torch.full((n, 64), float("nan"), device="cuda", dtype=BF)
         a2[:, :k2], b2[:, :k2] = rnd(m, k2), rnd(n, k2, 0.05)
         a2, b2 = a2[:, :k2], b2[:, :k2]
     bs = torch.randn(n, device="cuda", generator=g) if bias else None
@@ -34,3 +30,30 @@ def test_gemm_ksplit(m, n, k, k2, bias):
     bound = 2.0 ** -8 * want.abs() + (k + k2 + 16) * 2.0 ** -24 * (mag + 1.0)
     assert bool(((out[:m, :n].double() - want).abs() <= bound).all())
     assert bool((out[m] == 7.0).all()) and bool((out[:m, n:] == 7.0).all())
+    assert O.device_status() == 0
+
+
+@pytest.mark.parametrize("m,n,k,k2,bias", [
+    (512, 16, 13824, 0, False), (512, 48, 1152, 0, False), (129, 40, 2048, 0, False), (512, 1152, 13824, 32, False), (512, 1536, 1152, 48, False),
+    (1, 64, 4096, 0, False), (1, 8, 4104, 0, True), (129, 72, 1352, 16, True), (437, 640, 2048, 8, False), (437, 8, 2048, 0, False), (512, 2304, 768, 8, True),
+    (65, 128, 1000, 0, True), (1170, 896, 4864, 0, False), (300, 200, 1160, 64, True), (512, 50, 6912, 0, True), (1000, 768, 3072, 0, False)])
+def test_gemm_ksplit(m, n, k, k2, bias):
+    from mobilefinetuner_b200 import ops as O
+    cols, ranges = O.gemm_nt_ksplit_plan(m, n, k, k2)
+    assert cols in (64, 128) and 2 <= ranges <= 8, "the shape no longer reaches the K-split kernel"
+    _check(m, n, k, k2, bias)
+
+
+@pytest.mark.parametrize("m,n,k,k2", [(2100, 2200, 640, 16), (2305, 2000, 1152, 0), (4097, 1160, 264, 8)])
+def test_pair_kernel_ragged_bf16(m, n, k, k2):
+    """Ragged bf16 outputs of many tiles: the K-split kernel leaves them to 256-wide pair tiles."""
+    from mobilefinetuner_b200 import ops as O
+    assert O.gemm_nt_ksplit_plan(m, n, k, k2) == (0, 1) and O.gemm_nt_tile_cols(m, n, k, k2) == 256
+    _check(m, n, k, k2, True)
+
+
+@pytest.mark.parametrize("m,n,k,k2,bias", [(130, 40, 520, 0, False), (1, 64, 704, 0, False), (437, 8, 640, 0, False), (1985, 896, 4864, 0, False)])
+def test_shapes_of_the_other_kernels(m, n, k, k2, bias):
+    from mobilefinetuner_b200 import ops as O
+    assert O.gemm_nt_ksplit_plan(m, n, k, k2) == (0, 1)
+    _check(m, n, k, k2, bias)
