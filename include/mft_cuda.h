@@ -299,7 +299,8 @@ int32_t mft_accumulate_blocks_f32(const mft_block_copy_t* table_dev, int32_t n_e
  *             the saved gate|up tile and writes dgu[m, 2*inter] = (d_gate | d_up) directly.  w_kn = K-major [inter, k].
  * Both return MFT_ERR_UNSUPPORTED (without an error message) when the shape does not qualify (m < 256, inter not a
  * multiple of 128 / 64, unaligned operands): the caller then runs mft_gemm_nt followed by mft_act_fwd / mft_act_bwd,
- * whose results these calls reproduce bit for bit. */
+ * whose results these calls reproduce bit for bit (where mft_gemm_nt_ksplit_plan names that product they are those two
+ * launches; a backward call whose dgu overlaps gu stays in one and differs by the order of the f32 sums). */
 int32_t mft_glu_linear_fwd(int32_t kind, const void* x_bf16, int64_t ldx, const void* w_nk_bf16, int64_t ldw, int64_t m,
                            int64_t inter, int64_t k, const void* xa_bf16, int64_t ldxa, const void* b_nk_bf16, int64_t ldb2,
                            int64_t k2, const float* bias, void* gu_bf16, int64_t ld_gu, void* act_bf16, int64_t ld_act,

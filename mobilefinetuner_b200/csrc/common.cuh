@@ -71,6 +71,11 @@ cudaError_t launch_dep(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// mft_act_fwd / _bwd with a row stride for every operand (elementwise.cu); dy may be dup
+int32_t act_fwd_rows(int32_t kind, const void* gate, const void* up, int64_t ld, void* y, int64_t ldy, int64_t rows, int64_t cols, cudaStream_t st);
+int32_t act_bwd_rows(int32_t kind, const void* dy, int64_t lddy, const void* gate, const void* up, int64_t ld, void* dgate, void* dup, int64_t ldd,
+                     int64_t rows, int64_t cols, cudaStream_t st);
+
 #define MFT_CHECK_ARG(cond, msg)                                   \
     do {                                                           \
         if (!(cond)) return ::mft::fail(MFT_ERR_INVALID_ARG, msg); \

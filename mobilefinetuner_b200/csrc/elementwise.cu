@@ -107,7 +107,7 @@ __global__ void embedding_kernel(const int32_t* __restrict__ ids, const __nv_bfl
 // ---------------------------------------------------------------- activations
 template <int KIND>
 __global__ void act_fwd_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ up,
-                               int64_t ld, __nv_bfloat16* __restrict__ y, int64_t rows, int64_t cols) {
+                               int64_t ld, __nv_bfloat16* __restrict__ y, int64_t ldy, int64_t rows, int64_t cols) {
     dep_trigger();
     dep_wait();
     const int64_t vpr = cols / 8;
@@ -123,13 +123,14 @@ __global__ void act_fwd_kernel(const __nv_bfloat16* __restrict__ gate, const __n
             if (KIND == MFT_ACT_GELU) o[j] = gelu_tanh_fast(g[j]);
             else o[j] = glu_fwd(KIND == MFT_ACT_GEGLU, g[j], u[j]);
         }
-        store8(y + r * cols + c, o);
+        store8(y + r * ldy + c, o);
     }
 }
+// dy may be dup: a thread reads its columns of dy before it writes them to dup, and nobody else touches them
 template <int KIND>
-__global__ void act_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ gate,
+__global__ void act_bwd_kernel(const __nv_bfloat16* dy, int64_t lddy, const __nv_bfloat16* __restrict__ gate,
                                const __nv_bfloat16* __restrict__ up, int64_t ld,
-                               __nv_bfloat16* __restrict__ dgate, __nv_bfloat16* __restrict__ dup,
+                               __nv_bfloat16* __restrict__ dgate, __nv_bfloat16* dup, int64_t ldd,
                                int64_t rows, int64_t cols) {
     dep_trigger();
     dep_wait();
@@ -140,7 +141,7 @@ __global__ void act_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_
         const int64_t r = i / vpr, c = (i % vpr) * 8;
         float g[8], u[8], d[8], dg[8], du[8];
         load8(gate + r * ld + c, g);
-        load8(dy + r * cols + c, d);
+        load8(dy + r * lddy + c, d);
         if (KIND != MFT_ACT_GELU) load8(up + r * ld + c, u);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -152,8 +153,8 @@ __global__ void act_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_
                 glu_bwd(KIND == MFT_ACT_GEGLU, d[j], g[j], u[j], dg[j], du[j]);     // the same code as the GEMM epilogue that fuses it
             }
         }
-        store8(dgate + r * ld + c, dg);
-        if (KIND != MFT_ACT_GELU) store8(dup + r * ld + c, du);
+        store8(dgate + r * ldd + c, dg);
+        if (KIND != MFT_ACT_GELU) store8(dup + r * ldd + c, du);
     }
 }
 
@@ -288,6 +289,34 @@ __global__ void adam_kernel(float* __restrict__ p, float* __restrict__ g, float*
     }
 }
 
+int32_t act_fwd_rows(int32_t kind, const void* gate, const void* up, int64_t ld, void* y, int64_t ldy, int64_t rows, int64_t cols, cudaStream_t st) {
+    MFT_CHECK_ARG(gate && y && rows > 0 && cols > 0 && cols % 8 == 0 && ld % 8 == 0, "mft_act_fwd: bad argument (cols and ld must be multiples of 8)");
+    MFT_CHECK_ARG(kind == MFT_ACT_GELU || up, "mft_act_fwd: gated activation needs `up`");
+    const int g = grid_for(rows * cols / 8, 256);
+    auto G = (const __nv_bfloat16*)gate; auto U = (const __nv_bfloat16*)up; auto Y = (__nv_bfloat16*)y;
+    if (kind == MFT_ACT_GELU) launch_dep(act_fwd_kernel<MFT_ACT_GELU>, dim3(g), dim3(256), (size_t)(0), st, G, U, ld, Y, ldy, rows, cols);
+    else if (kind == MFT_ACT_SWIGLU) launch_dep(act_fwd_kernel<MFT_ACT_SWIGLU>, dim3(g), dim3(256), (size_t)(0), st, G, U, ld, Y, ldy, rows, cols);
+    else if (kind == MFT_ACT_GEGLU) launch_dep(act_fwd_kernel<MFT_ACT_GEGLU>, dim3(g), dim3(256), (size_t)(0), st, G, U, ld, Y, ldy, rows, cols);
+    else return fail(MFT_ERR_INVALID_ARG, "mft_act_fwd: unknown kind");
+    MFT_LAUNCH_CHECK("act_fwd");
+    return MFT_OK;
+}
+
+int32_t act_bwd_rows(int32_t kind, const void* dy, int64_t lddy, const void* gate, const void* up, int64_t ld, void* dgate, void* dup, int64_t ldd,
+                     int64_t rows, int64_t cols, cudaStream_t st) {
+    MFT_CHECK_ARG(dy && gate && dgate && rows > 0 && cols > 0 && cols % 8 == 0 && ld % 8 == 0, "mft_act_bwd: bad argument");
+    MFT_CHECK_ARG(kind == MFT_ACT_GELU || (up && dup), "mft_act_bwd: gated activation needs `up` and `dup`");
+    const int g = grid_for(rows * cols / 8, 256);
+    auto D = (const __nv_bfloat16*)dy; auto G = (const __nv_bfloat16*)gate; auto U = (const __nv_bfloat16*)up;
+    auto DG = (__nv_bfloat16*)dgate; auto DU = (__nv_bfloat16*)dup;
+    if (kind == MFT_ACT_GELU) launch_dep(act_bwd_kernel<MFT_ACT_GELU>, dim3(g), dim3(256), (size_t)(0), st, D, lddy, G, U, ld, DG, DU, ldd, rows, cols);
+    else if (kind == MFT_ACT_SWIGLU) launch_dep(act_bwd_kernel<MFT_ACT_SWIGLU>, dim3(g), dim3(256), (size_t)(0), st, D, lddy, G, U, ld, DG, DU, ldd, rows, cols);
+    else if (kind == MFT_ACT_GEGLU) launch_dep(act_bwd_kernel<MFT_ACT_GEGLU>, dim3(g), dim3(256), (size_t)(0), st, D, lddy, G, U, ld, DG, DU, ldd, rows, cols);
+    else return fail(MFT_ERR_INVALID_ARG, "mft_act_bwd: unknown kind");
+    MFT_LAUNCH_CHECK("act_bwd");
+    return MFT_OK;
+}
+
 }  // namespace mft
 
 using namespace mft;
@@ -341,30 +370,11 @@ int32_t mft_embedding_gather(const int32_t* ids, const void* table, const void* 
 
 int32_t mft_act_fwd(int32_t kind, const void* gate, const void* up, int64_t ld, void* y, int64_t rows, int64_t cols,
                     mft_stream_t stream) {
-    MFT_CHECK_ARG(gate && y && rows > 0 && cols > 0 && cols % 8 == 0 && ld % 8 == 0, "mft_act_fwd: bad argument (cols and ld must be multiples of 8)");
-    MFT_CHECK_ARG(kind == MFT_ACT_GELU || up, "mft_act_fwd: gated activation needs `up`");
-    const int g = grid_for(rows * cols / 8, 256);
-    auto G = (const __nv_bfloat16*)gate; auto U = (const __nv_bfloat16*)up; auto Y = (__nv_bfloat16*)y;
-    if (kind == MFT_ACT_GELU) launch_dep(act_fwd_kernel<MFT_ACT_GELU>, dim3(g), dim3(256), (size_t)(0), as_stream(stream), G, U, ld, Y, rows, cols);
-    else if (kind == MFT_ACT_SWIGLU) launch_dep(act_fwd_kernel<MFT_ACT_SWIGLU>, dim3(g), dim3(256), (size_t)(0), as_stream(stream), G, U, ld, Y, rows, cols);
-    else if (kind == MFT_ACT_GEGLU) launch_dep(act_fwd_kernel<MFT_ACT_GEGLU>, dim3(g), dim3(256), (size_t)(0), as_stream(stream), G, U, ld, Y, rows, cols);
-    else return fail(MFT_ERR_INVALID_ARG, "mft_act_fwd: unknown kind");
-    MFT_LAUNCH_CHECK("act_fwd");
-    return MFT_OK;
+    return act_fwd_rows(kind, gate, up, ld, y, cols, rows, cols, as_stream(stream));
 }
 int32_t mft_act_bwd(int32_t kind, const void* dy, const void* gate, const void* up, int64_t ld, void* dgate, void* dup,
                     int64_t rows, int64_t cols, mft_stream_t stream) {
-    MFT_CHECK_ARG(dy && gate && dgate && rows > 0 && cols > 0 && cols % 8 == 0 && ld % 8 == 0, "mft_act_bwd: bad argument");
-    MFT_CHECK_ARG(kind == MFT_ACT_GELU || (up && dup), "mft_act_bwd: gated activation needs `up` and `dup`");
-    const int g = grid_for(rows * cols / 8, 256);
-    auto D = (const __nv_bfloat16*)dy; auto G = (const __nv_bfloat16*)gate; auto U = (const __nv_bfloat16*)up;
-    auto DG = (__nv_bfloat16*)dgate; auto DU = (__nv_bfloat16*)dup;
-    if (kind == MFT_ACT_GELU) launch_dep(act_bwd_kernel<MFT_ACT_GELU>, dim3(g), dim3(256), (size_t)(0), as_stream(stream), D, G, U, ld, DG, DU, rows, cols);
-    else if (kind == MFT_ACT_SWIGLU) launch_dep(act_bwd_kernel<MFT_ACT_SWIGLU>, dim3(g), dim3(256), (size_t)(0), as_stream(stream), D, G, U, ld, DG, DU, rows, cols);
-    else if (kind == MFT_ACT_GEGLU) launch_dep(act_bwd_kernel<MFT_ACT_GEGLU>, dim3(g), dim3(256), (size_t)(0), as_stream(stream), D, G, U, ld, DG, DU, rows, cols);
-    else return fail(MFT_ERR_INVALID_ARG, "mft_act_bwd: unknown kind");
-    MFT_LAUNCH_CHECK("act_bwd");
-    return MFT_OK;
+    return act_bwd_rows(kind, dy, cols, gate, up, ld, dgate, dup, ld, rows, cols, as_stream(stream));
 }
 int32_t mft_add_f32(const float* a, const float* b, float* out, int64_t n, mft_stream_t stream) {
     MFT_CHECK_ARG(a && b && out && n > 0, "mft_add_f32: bad argument");

@@ -492,8 +492,33 @@ static bool gemm_ksplit_enabled() {
     return use_clusters && device_status_word();
 }
 
+// A gated-MLP call is promised to have the bits of the plain product followed by the activation kernel.  The pair kernel's
+// epilogue has them where the plain call runs on pair tiles; where that call goes to the K-split kernel, whose sums run in
+// another order, the two launches themselves take its place.  d(act) waits in the half of D where d_up will be, so D must
+// not be the saved gate|up (such a call stays on the pair kernel).
+static int32_t gemm_nt_run_glu_in_two(const GemmCall& c, cudaStream_t stream) {
+    if (!gemm_nt_pair_takes(c)) return MFT_ERR_UNSUPPORTED;
+    const bool fwd = c.epi == EPI_GLU_FWD;
+    const int64_t I = c.glu_inter;
+    const int32_t kind = c.glu_geglu ? MFT_ACT_GEGLU : MFT_ACT_SWIGLU;
+    auto* d = static_cast<__nv_bfloat16*>(c.d);
+    auto* aux = static_cast<__nv_bfloat16*>(c.aux);
+    if (!fwd && d < aux + (c.m - 1) * c.ld_aux + 2 * I && aux < d + (c.m - 1) * c.ldd + 2 * I) return MFT_ERR_UNSUPPORTED;
+    GemmCall plain = c;
+    plain.epi = EPI_STORE;
+    plain.aux = nullptr;
+    if (!fwd) plain.d = d + I;
+    if (int32_t s = gemm_nt_run_ksplit(plain, stream)) return s;
+    return fwd ? act_fwd_rows(kind, d, d + I, c.ldd, aux, c.ld_aux, c.m, I, stream)
+               : act_bwd_rows(kind, d + I, c.ldd, aux, aux + I, c.ld_aux, d, d + I, c.ldd, c.m, I, stream);
+}
+
 static int32_t gemm_nt_run_inner(const GemmCall& c, cudaStream_t stream) {
     if (gemm_ksplit_enabled()) {
+        if (c.epi == EPI_GLU_FWD || c.epi == EPI_GLU_BWD) {
+            const int32_t s0 = gemm_nt_run_glu_in_two(c, stream);
+            if (s0 != MFT_ERR_UNSUPPORTED) return s0;
+        }
         const int32_t s1 = gemm_nt_run_ksplit(c, stream);
         if (s1 != MFT_ERR_UNSUPPORTED) return s1;
         const int32_t s2 = gemm_nt_run_2cta(c, stream);

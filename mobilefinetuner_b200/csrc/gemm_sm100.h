@@ -92,6 +92,7 @@ __host__ __device__ inline int tile_n(int tile, const GemmParams& p) {
 int32_t gemm_nt_run(const GemmCall& c, cudaStream_t stream);
 // CTA-pair (cta_group::2) variant for 256 x 256 cluster tiles; returns MFT_ERR_UNSUPPORTED when the call does not qualify.
 int32_t gemm_nt_run_2cta(const GemmCall& c, cudaStream_t stream);
+bool gemm_nt_pair_takes(const GemmCall& c);       // what it asks of a call before it builds tensor maps
 // K-split variant for bf16 outputs of few tiles (gemm_ksplit.cu); MFT_ERR_UNSUPPORTED when the call does not qualify or
 // another kernel is the faster one.
 struct KsplitPlan { int bn = 0, splits = 1; };

@@ -456,23 +456,27 @@ int gemm_nt_pair_tile_cols(int64_t m, int64_t n, int64_t k, int64_t k2, bool d_i
     return plan_tiles(m, (n + 255) / 256, n >= 384 ? (n + 383) / 384 : 0, kb, !d_is_f32, d_is_f32 && k2 == 0, 0, &splits, n % 384 != 0);
 }
 
-int32_t gemm_nt_run_2cta(const GemmCall& c, cudaStream_t stream) {
+bool gemm_nt_pair_takes(const GemmCall& c) {
     const bool ce = c.epi == EPI_CE_GRAD || c.epi == EPI_CE_P;
     const bool glu = c.epi == EPI_GLU_FWD || c.epi == EPI_GLU_BWD;
     const bool bf16_ok = !c.d_is_f32 && !c.accumulate && (c.ldd % 8 == 0);
     const bool f32_ok = c.d_is_f32 && c.epi == EPI_STORE && (c.ldd % 4 == 0);
     const bool ok = (c.epi == EPI_STORE || ce || glu) && (bf16_ok || f32_ok) && c.d && (reinterpret_cast<uintptr_t>(c.d) % 16 == 0) &&
                     c.m >= 256 && c.n >= 192 && c.splits >= 0 && c.splits <= 64;
-    if (!ok) return MFT_ERR_UNSUPPORTED;
+    if (!ok) return false;
     if (glu) {
         // forward: n = 2 * inter columns of D, tiles of 128 gate + 128 up columns; backward: n = inter
         const int64_t inter = c.glu_inter;
         const bool shape_ok = c.epi == EPI_GLU_FWD ? (c.n == 2 * inter && inter % 128 == 0) : (c.n == inter && inter % 64 == 0);
         if (!shape_ok || !c.aux || c.ld_aux % 8 != 0 || reinterpret_cast<uintptr_t>(c.aux) % 16 != 0 || c.d_is_f32 || inter >= (1 << 30))
-            return MFT_ERR_UNSUPPORTED;
+            return false;
     }
-    const bool can_split = f32_ok && c.k2 == 0;
-    if (c.splits > 1 && !can_split) return MFT_ERR_UNSUPPORTED;
+    return c.splits <= 1 || (f32_ok && c.k2 == 0);
+}
+
+int32_t gemm_nt_run_2cta(const GemmCall& c, cudaStream_t stream) {
+    if (!gemm_nt_pair_takes(c)) return MFT_ERR_UNSUPPORTED;
+    const bool bf16_ok = !c.d_is_f32, can_split = c.d_is_f32 && c.k2 == 0;
     const int64_t kb = (c.k + BK - 1) / BK + (c.k2 > 0 ? 1 : 0);
     // the wide tile: plain store or gated-MLP forward over whole 384-column tiles, when the cost model prefers it (a call
     // of a few tiles is one wave either way, and the wave of wide tiles is the longer one)

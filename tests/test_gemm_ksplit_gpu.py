@@ -57,3 +57,48 @@ def test_shapes_of_the_other_kernels(m, n, k, k2, bias):
     from mobilefinetuner_b200 import ops as O
     assert O.gemm_nt_ksplit_plan(m, n, k, k2) == (0, 1)
     _check(m, n, k, k2, bias)
+
+
+# the gated-MLP calls have the bits of the plain product and the activation kernel, also where that product is K-split;
+# gate|up and its gradient with row strides of their own
+@pytest.mark.parametrize("swiglu", [False, True])
+@pytest.mark.parametrize("m,inter,k,r", [(512, 2048, 640, 0), (512, 2048, 640, 16), (257, 448, 1160, 16), (300, 256, 2048, 0)])
+def test_gated_mlp_calls_keep_the_bits(swiglu, m, inter, k, r):
+    from mobilefinetuner_b200 import _lib as L
+    from mobilefinetuner_b200 import ops as O
+    kind = L.ACT_SWIGLU if swiglu else L.ACT_GEGLU
+    g = torch.Generator(device="cuda").manual_seed(m + inter)
+    st = torch.cuda.current_stream().cuda_stream
+
+    def rnd(rows, cols, scale=1.0):
+        return (torch.randn(rows, cols, device="cuda", generator=g) * scale).to(BF)
+    dy, wd, gu_wide = rnd(m, k), rnd(inter, k, 0.05), rnd(m, 2 * inter + 16)
+    gu = gu_wide[:, :2 * inter]
+    a2, b2 = (rnd(m, 64)[:, :r], rnd(inter, 64, 0.05)[:, :r]) if r else (None, None)
+    assert O.gemm_nt_ksplit_plan(m, inter, k, r)[0] > 0
+
+    def bwd(gu, dgu):
+        L.call("mft_glu_linear_bwd", kind, dy.data_ptr(), k, wd.data_ptr(), k, m, inter, k, a2.data_ptr() if r else None, 64, b2.data_ptr() if r else None,
+               64, r, gu.data_ptr(), gu.stride(0), dgu.data_ptr(), dgu.stride(0), st)
+    dgu_wide = torch.full((m + 1, 2 * inter + 8), 3.0, device="cuda", dtype=BF)
+    bwd(gu, dgu_wide[:m, :2 * inter])
+    dg, du = O.act_bwd(kind, O.gemm_nt(dy, wd, a2=a2, b2=b2), gu[:, :inter].contiguous(), gu[:, inter:].contiguous())
+    assert torch.equal(dgu_wide[:m, :inter], dg) and torch.equal(dgu_wide[:m, inter:2 * inter], du)
+    assert bool((dgu_wide[m] == 3.0).all()) and bool((dgu_wide[:, 2 * inter:] == 3.0).all())
+    # in place over the saved gate|up: taken as before, equal to the rounding of d(act) to bf16
+    both = gu.contiguous()
+    bwd(both, both)
+    for x, y in ((both[:, :inter], dg), (both[:, inter:], du)):
+        assert (x.float() - y.float()).norm() <= 2.0 ** -8 * y.float().norm()
+    # forward
+    if inter % 128 == 0 and O.gemm_nt_ksplit_plan(m, 2 * inter, k, r)[0] > 0:
+        x, w = dy, rnd(2 * inter, k, 0.05)
+        xa, bp = (rnd(m, 64)[:, :r], rnd(2 * inter, 64, 0.05)[:, :r]) if r else (None, None)
+        bias = torch.randn(2 * inter, device="cuda", generator=g)
+        gu_f, act_wide = torch.empty(m, 2 * inter + 8, device="cuda", dtype=BF)[:, :2 * inter], torch.full((m, inter + 8), 3.0, device="cuda", dtype=BF)
+        L.call("mft_glu_linear_fwd", kind, x.data_ptr(), k, w.data_ptr(), k, m, inter, k, xa.data_ptr() if r else None, 64, bp.data_ptr() if r else None, 64, r,
+               bias.data_ptr(), gu_f.data_ptr(), gu_f.stride(0), act_wide.data_ptr(), act_wide.stride(0), st)
+        want = O.gemm_nt(x, w, a2=xa, b2=bp, bias=bias)
+        assert torch.equal(gu_f, want) and torch.equal(act_wide[:, :inter], O.act_fwd(kind, want[:, :inter], want[:, inter:]))
+        assert bool((act_wide[:, inter:] == 3.0).all())
+    assert O.device_status() == 0
