@@ -111,8 +111,8 @@ gemm_nt_ksplit_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
 
     if (warp == 0) {
         if (lane == 0) {
-            int stage = 0, issued = 0; uint32_t phase = 0;
-            for (int kb = kb0; kb < kb1; ++kb, ++issued) {
+            int stage = 0; uint32_t phase = 0;
+            for (int kb = kb0; kb < kb1; ++kb) {
                 if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) break;
                 uint8_t* sa = tiles + stage * Cfg::STAGE_BYTES;
                 mbar_arrive_expect_tx(&full_bar[stage], Cfg::STAGE_BYTES);
@@ -122,8 +122,6 @@ gemm_nt_ksplit_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                 tma_load_2d(sa + Cfg::A_BYTES, main_kb ? &map_b : &map_b2, &full_bar[stage], k0, n0);
                 if (++stage == Cfg::STAGES) { stage = 0; phase ^= 1; }
             }
-            // the stages become the cluster's exchange area: no load of this CTA may land in them after a wait ran out
-            if (!mbar_wait(tmem_full_bar, 0, abort_flag)) drain_loads(full_bar, Cfg::STAGES, issued);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -132,7 +130,8 @@ gemm_nt_ksplit_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         // a ragged last column tile issues narrower MMAs (existing columns rounded up to 16)
         const uint32_t idesc = idesc_bf16_f32(BM, (uint32_t)min(BN, (p.n - n0 + 15) & ~15));
         const uint64_t desc0 = smem_desc_sw128(smem_u32(tiles));
-        for (int kb = kb0; kb < kb1; ++kb) {
+        int kb = kb0;
+        for (; kb < kb1; ++kb) {
             if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, abort_flag))) { ok = false; break; }
             tc_fence_after();
             const uint64_t adesc = desc0 + (uint64_t)(stage * (Cfg::STAGE_BYTES >> 4)), bdesc = adesc + (Cfg::A_BYTES >> 4);
@@ -149,6 +148,9 @@ gemm_nt_ksplit_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
             __syncwarp();
             if (++stage == Cfg::STAGES) { stage = 0; phase ^= 1; }
         }
+        // the stages become the cluster's exchange area: no load of this CTA may land in them after a wait ran out.  What can
+        // be in flight then are the loads from the k-block that did not come on, at most one per stage.
+        if (!ok) drain_loads(full_bar, Cfg::STAGES, kb - kb0, min(kb1 - kb0, kb - kb0 + Cfg::STAGES));
         if (ok && elect_one()) umma_commit(tmem_full_bar);
         __syncwarp();
     }

@@ -115,7 +115,7 @@ gemm_nt_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     ++issued;
                 }
             }
-            if (!ok) drain_loads(full_bar, Cfg::STAGES, issued);     // nothing may land after the CTA has left
+            if (!ok) drain_loads(full_bar, Cfg::STAGES, max(0, issued - Cfg::STAGES), issued);     // nothing may land after the CTA has left
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer (warp-uniform loop, one elected lane issues: see the pair kernel)

@@ -76,14 +76,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     }
 }
 
-// For a CTA that gives up: bounded wait for its own loads that may still be in flight.  `issued` loads were armed round robin
-// on the `stages` barriers of `full`; the last one on a stage completes that barrier's phase number (times armed - 1).
-__device__ __forceinline__ void drain_loads(uint64_t* full, int stages, int issued) {
+// For a CTA that gives up: bounded wait for its loads `from` .. `to` - 1 that may still be in flight (load i goes to stage
+// i % stages and completes phase i / stages of that stage's barrier).  Out of line, to keep it off the kernels' hot path.
+static __device__ __noinline__ void drain_loads(uint64_t* full, int stages, int from, int to) {
     const unsigned long long t0 = globaltimer_ns();
-    for (int s = 0; s < stages && s < issued; ++s) {
-        const uint32_t last = (uint32_t)((issued - 1 - s) / stages);
-        while (!mbar_try_wait(&full[s], last & 1u) && globaltimer_ns() - t0 < WAIT_LIMIT_NS) {}
-    }
+    for (int i = from; i < to; ++i)
+        while (!mbar_try_wait(&full[i % stages], (uint32_t)(i / stages) & 1u) && globaltimer_ns() - t0 < WAIT_LIMIT_NS) {}
 }
 
 // ---- TMA (2-D tiled load into this CTA's shared memory)
