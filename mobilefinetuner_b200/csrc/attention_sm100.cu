@@ -242,15 +242,16 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         // (The tensor pipe takes MMAs from a thread only about as fast as that thread issues them: every wait,
         // fence and commit between two MMAs is exposed when the MMAs are short.  Two issuing threads overlap
         // one product's bookkeeping with the other product's MMAs.)
-        constexpr uint32_t idesc_s = idesc_bf16_f32(BM, BN);
-        bool ok = warp_wait(q_full, 0, abort_flag);
-        const uint64_t qd = smem_desc_sw128(smem_u32(q_smem));
-        for (int t = 0; t < n_tiles && ok; ++t) {
-            const int st = t & 1;
-            const uint32_t ph = (t >> 1) & 1;
-            if (!warp_wait(&k_full[st], ph, abort_flag) || !warp_wait(&s_free[st], ph ^ 1, abort_flag)) { ok = false; break; }
-            tc_fence_after();
-            if (elect_one()) {
+        {
+            constexpr uint32_t idesc_s = idesc_bf16_f32(BM, BN);
+            bool ok = warp_wait(q_full, 0, abort_flag);
+            const uint64_t qd = smem_desc_sw128(smem_u32(q_smem));
+            for (int t = 0; t < n_tiles && ok; ++t) {
+                const int st = t & 1;
+                const uint32_t ph = (t >> 1) & 1;
+                if (!warp_wait(&k_full[st], ph, abort_flag) || !warp_wait(&s_free[st], ph ^ 1, abort_flag)) { ok = false; break; }
+                tc_fence_after();
+                if (elect_one()) {
                 const uint64_t kd = smem_desc_sw128(smem_u32(k_smem + st * KV_BYTES));
                 const uint32_t tmem_s = tmem_base + S_COL + st * BN;
 #pragma unroll
@@ -261,21 +262,23 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                                   (c | j) != 0 ? 1u : 0u);
                 umma_commit(&k_empty[st]);
                 umma_commit(&s_full[st]);
+                }
+                __syncwarp();
             }
-            __syncwarp();
         }
     } else if (warp == 10) {
         // ------------------------------------------------ MMA issuer 2: O += P V
-        constexpr uint32_t idesc_o = idesc_bf16_f32(BM, HD) | IDESC_B_MN;
-        bool ok = true;
-        int vs = 0;
-        uint32_t vph = 0;
-        for (int t = 0; t < n_tiles && ok; ++t) {
-            const int st = t & 1;
-            const uint32_t ph = (t >> 1) & 1;
-            if (!warp_wait(&v_full[vs], vph, abort_flag) || !warp_wait(&p_full[st], ph, abort_flag)) { ok = false; break; }
-            tc_fence_after();
-            if (elect_one()) {
+        {
+            constexpr uint32_t idesc_o = idesc_bf16_f32(BM, HD) | IDESC_B_MN;
+            bool ok = true;
+            int vs = 0;
+            uint32_t vph = 0;
+            for (int t = 0; t < n_tiles && ok; ++t) {
+                const int st = t & 1;
+                const uint32_t ph = (t >> 1) & 1;
+                if (!warp_wait(&v_full[vs], vph, abort_flag) || !warp_wait(&p_full[st], ph, abort_flag)) { ok = false; break; }
+                tc_fence_after();
+                if (elect_one()) {
                 // A = the bf16 probabilities in tensor memory (8 columns per 16 keys), B = V as it lies in memory
                 const uint32_t pa = tmem_base + P_COL + st * 32;
                 const uint64_t vd = smem_desc_mn_sw128(smem_u32(v_smem + vs * KV_BYTES), BN * 128);
@@ -285,9 +288,10 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 umma_commit(&v_empty[vs]);
                 umma_commit(&p_free[st]);
                 umma_commit(&o_done[st]);
+                }
+                __syncwarp();
+                if (++vs == FWD_VST) { vs = 0; vph ^= 1; }
             }
-            __syncwarp();
-            if (++vs == FWD_VST) { vs = 0; vph ^= 1; }
         }
     } else {
         // ------------------------------------------------ softmax (warps 2..9): two threads per query row (32 keys each)
@@ -428,7 +432,7 @@ constexpr int DQ_S_COL = 0, DQ_DP_COL = 64, DQ_ACC_COL = 128;
 template <int HD>
 struct DqDim {
     static constexpr int KV_BYTES = DQ_BN * HD * 2;    // CH chunks of [32 rows x 64 columns]
-    static constexpr int SMEM = 2 * Dim<HD>::Q_BYTES + (DQ_KST + DQ_VST) * KV_BYTES + 256;
+    static constexpr int SMEM = 2 * Dim<HD>::Q_BYTES + (DQ_KST + DQ_VST) * KV_BYTES + 256 + 4 * BM * 4;
     static constexpr int DS_COL = 128 + HD;            // dS as the A operand of the dQ product: 16 columns (32 keys as bf16 pairs) per group
     static constexpr int TMEM = HD == 64 ? 256 : 512;
     static constexpr int GROUPS = HD == 64 ? 1 : 2;
@@ -447,6 +451,10 @@ struct BwdParams {
     float* dkv_acc;
     int32_t* status;
     int q_col0_stride, do_col0_stride, k_col0_stride, v_col0_stride;
+    // dQ kernel only: when o != nullptr the kernel first forms delta[row] = sum_d O * dO for its rows and stores it
+    const __nv_bfloat16 *o, *d_o;
+    long long so_b, so_s, so_h, sdo_b, sdo_s, sdo_h;
+    float* delta_out;
 };
 
 template <int HD, bool RAGGED>
@@ -474,6 +482,7 @@ attn_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     uint64_t* acc_done = bars + 21;     // [1]  completed once, by the last dQ product
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    float* delta_smem = reinterpret_cast<float*>(bars + 32);   // [4][128] partial rowsum(O * dO) of this CTA's queries
     if ((smem_u32(smem_raw) & 1023u) != 0) {
         if (threadIdx.x == 0 && p.status) atomicExch(p.status, MFT_ERR_INVALID_ARG);
         return;
@@ -586,7 +595,32 @@ attn_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         const int ic = RAGGED ? min(i, p.seq - 1) : i; // rows past the end: a valid row's numbers, nothing of theirs is stored
         const long long sidx = ((long long)b * p.n_heads + h) * p.seq + ic;
         const float neg_lse2 = -p.lse[sidx] * LOG2E;
-        const float dlt = p.delta[sidx];
+        float dlt;
+        if (HD == 256 && p.o != nullptr) {
+            // delta = rowsum(O * dO): the four element-wise threads of a row (2 groups x 2 halves) take 64 columns
+            // each, the partial sums meet in shared memory; thread (group 0, half 0) stores the row's delta for the
+            // dK/dV kernel
+            {
+                const int part = g0 * 2 + half;
+                const __nv_bfloat16* orow = p.o + (long long)b * p.so_b + (long long)ic * p.so_s + (long long)h * p.so_h + part * 64;
+                const __nv_bfloat16* drow = p.d_o + (long long)b * p.sdo_b + (long long)ic * p.sdo_s + (long long)h * p.sdo_h + part * 64;
+                float a8[8][8], c8[8][8];
+#pragma unroll
+                for (int d = 0; d < 8; ++d) { load8(orow + d * 8, a8[d]); load8(drow + d * 8, c8[d]); }
+                float acc = 0.f;
+#pragma unroll
+                for (int d = 0; d < 8; ++d)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) acc = fmaf(a8[d][e], c8[d][e], acc);
+                delta_smem[part * BM + r] = acc;
+            }
+            asm volatile("bar.sync 1, 512;" ::: "memory");     // the 16 element-wise warps
+            const float dsum = (delta_smem[r] + delta_smem[BM + r]) + (delta_smem[2 * BM + r] + delta_smem[3 * BM + r]);
+            if (g0 == 0 && half == 0 && i < p.seq) p.delta_out[sidx] = dsum;
+            dlt = dsum;
+        } else {
+            dlt = p.delta[sidx];
+        }
         bool ok = true;
         for (int t = g0; t < n_tiles && ok; t += GROUPS) {
             const int g = t & 1;                       // tensor-memory buffer of the tile
@@ -1058,10 +1092,11 @@ static int32_t box_map(CUtensorMap* map, const void* base, const AttnParams& a, 
                       : make_tmap_bf16(map, base, (int64_t)a.batch * a.seq, cols, ld, box_rows);
 }
 
-int32_t attn_dq_sm100(const AttnParams& a, int hd, cudaStream_t stream) {
+int32_t attn_dq_sm100(const AttnParams& a, int hd, bool compute_delta, cudaStream_t stream) {
     static const int enabled = [] { const char* e = std::getenv("MFT_ATTN_TC"); return e ? std::atoi(e) : 1; }();
     if (!enabled || !tc_shape_ok(hd) || !device_status_word()) return MFT_ERR_UNSUPPORTED;
     if (!bwd_long_enough(hd, a.seq) && enabled < 2) return MFT_ERR_UNSUPPORTED;
+    if (compute_delta && hd != 256) return MFT_ERR_UNSUPPORTED;
     if (!aligned16(a.dq)) return MFT_ERR_UNSUPPORTED;
     if (!token_major(a.sq, a.seq) || !token_major(a.sk, a.seq) || !token_major(a.sv, a.seq) || !token_major(a.sdo, a.seq)) return MFT_ERR_UNSUPPORTED;
     if (a.sq.stride_h % 8 || a.sk.stride_h % 8 || a.sv.stride_h % 8 || a.sdo.stride_h % 8) return MFT_ERR_UNSUPPORTED;
@@ -1077,6 +1112,12 @@ int32_t attn_dq_sm100(const AttnParams& a, int hd, cudaStream_t stream) {
     p.dkv_acc = a.dkv_acc; p.status = device_status_word();
     p.q_col0_stride = (int)a.sq.stride_h; p.do_col0_stride = (int)a.sdo.stride_h;
     p.k_col0_stride = (int)a.sk.stride_h; p.v_col0_stride = (int)a.sv.stride_h;
+    if (compute_delta) {
+        if (a.so.stride_b % 8 || a.so.stride_s % 8 || a.so.stride_h % 8 || a.sdo.stride_b % 8 || a.sdo.stride_s % 8) return MFT_ERR_UNSUPPORTED;
+        p.o = a.o; p.d_o = a.d_o; p.delta_out = a.delta;
+        p.so_b = a.so.stride_b; p.so_s = a.so.stride_s; p.so_h = a.so.stride_h;
+        p.sdo_b = a.sdo.stride_b; p.sdo_s = a.sdo.stride_s; p.sdo_h = a.sdo.stride_h;
+    }
     dim3 grid((unsigned)((a.seq + BM - 1) / BM), (unsigned)a.n_heads, (unsigned)a.batch);
     return HD_DISPATCH(hd, launch_dq<64>(mq, md, mk, mv, p, grid, stream), launch_dq<128>(mq, md, mk, mv, p, grid, stream), launch_dq<256>(mq, md, mk, mv, p, grid, stream));
 }
