@@ -20,6 +20,8 @@
 // Tensor-core path: warp-level mma.sync m16n8k16 (bf16 in, fp32 accumulate).
 #include "common.cuh"
 
+#include <cooperative_groups.h>
+
 #include <cstdlib>
 
 #include "attention.h"
@@ -27,6 +29,8 @@
 namespace mft {
 
 namespace {
+
+namespace cg = cooperative_groups;
 
 constexpr float LOG2E = 1.4426950408889634f;
 
@@ -384,9 +388,14 @@ attn_bwd_dq_kernel(const AttnParams p) {
 // [wn*HD/WN, (wn+1)*HD/WN).  S^T and dP^T (keys x queries) are computed with the
 // 64 queries split across the WN warps of a row, written to shared memory as
 // bf16 and re-read as the A operand of the two accumulating products.
-// SPLIT = false: grid.y = KV heads, the CTA walks all query heads of its group and stores bf16 dK/dV.
-// SPLIT = true : grid.y = query heads, the CTA adds its head's contribution into the f32 accumulator.
-template <int HD, int WN, bool SPLIT>
+// Heads::kWhole  : grid.y = KV heads, the CTA walks all query heads of its group and stores bf16 dK/dV.
+// Heads::kAtomic : grid.y = query heads, the CTA adds its head's contribution into the f32 accumulator.
+// Heads::kCluster: grid.y = query heads, the CTAs of a group are a cluster.  Each leaves its f32 tile in its shared memory and
+//                  every one adds its share of the rows over all heads, in head order, and stores bf16: no accumulator to
+//                  clear and convert, and the sum does not depend on timing.
+constexpr int dkv_smem_bytes(int hd) { return 6 * 64 * (hd + 8) * 2 + 2 * 64 * (64 + 8) * 2 + 4 * 64 * 4; }
+enum class Heads { kWhole, kAtomic, kCluster };
+template <int HD, int WN, Heads HEADS>
 __global__ void __launch_bounds__(128 * WN)
 attn_bwd_dkv_kernel(const AttnParams p) {
     dep_trigger();
@@ -398,6 +407,7 @@ attn_bwd_dkv_kernel(const AttnParams p) {
     constexpr int DW = HD / WN;            // d-columns per warp
     constexpr int QW = BM / WN;            // queries per warp in the score products
     constexpr int STAGE = 2 * BM * LD;     // elements of one { Q, dO } stage
+    constexpr bool SPLIT = HEADS != Heads::kWhole;
     extern __shared__ __align__(16) uint8_t smem_attn[];
     __nv_bfloat16* Ks = reinterpret_cast<__nv_bfloat16*>(smem_attn);
     __nv_bfloat16* Vs = Ks + BN * LD;
@@ -515,11 +525,44 @@ attn_bwd_dkv_kernel(const AttnParams p) {
             }
         }
     }
+    if constexpr (HEADS == Heads::kCluster) {
+        constexpr int FLD = HD + 8;                                // row stride of the f32 tiles: eight rows of a warp on eight banks each
+        static_assert(2 * BN * FLD * 4 <= dkv_smem_bytes(HD), "the partial tiles take the place of the operands");
+        cg::cluster_group cluster = cg::this_cluster();
+        float* part = reinterpret_cast<float*>(smem_attn);         // [dK | dV][64 keys][FLD]
+        __syncthreads();                                           // every warp is done with the operands
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            float* krow = part + (wm * 16 + g + r * 8) * FLD + wn * DW + tq * 2;
+            float* vrow = krow + BN * FLD;
+#pragma unroll
+            for (int db = 0; db < DW / 8; ++db) {
+                *reinterpret_cast<float2*>(krow + db * 8) = make_float2(dk[db][r * 2] * p.scale, dk[db][r * 2 + 1] * p.scale);
+                *reinterpret_cast<float2*>(vrow + db * 8) = make_float2(dv[db][r * 2], dv[db][r * 2 + 1]);
+            }
+        }
+        cluster.sync();
+        for (int u = (int)cluster.block_rank() * THREADS + threadIdx.x; u < 2 * BN * (HD / 4); u += p.rep * THREADS) {
+            const int row = u / (HD / 4), d = (u % (HD / 4)) * 4, j = j0 + row % BN;       // rows 0..63 dK, 64..127 dV
+            if (j >= p.seq) continue;
+            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int c = 0; c < p.rep; ++c) {
+                const float4 x = *reinterpret_cast<const float4*>(cluster.map_shared_rank(part, c) + row * FLD + d);
+                s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
+            }
+            const mft_strides_t& ss = row < BN ? p.sk : p.sv;
+            uint32_t* out = reinterpret_cast<uint32_t*>((row < BN ? p.dk : p.dv) + (int64_t)b * ss.stride_b + (int64_t)j * ss.stride_s + (int64_t)kvh * ss.stride_h + d);
+            out[0] = pack_bf16(s.x, s.y);
+            out[1] = pack_bf16(s.z, s.w);
+        }
+        cluster.sync();                                            // nobody leaves while its tile is still being read
+        return;
+    }
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
         const int j = j0 + wm * 16 + g + r * 8;
         if (j < p.seq) {
-            if constexpr (SPLIT) {
+            if constexpr (HEADS == Heads::kAtomic) {
                 const int64_t half = (int64_t)p.batch * p.seq * p.n_kv * HD;
                 float* krow = p.dkv_acc + (((int64_t)b * p.seq + j) * p.n_kv + kvh) * HD + wn * DW;
                 float* vrow = krow + half;
@@ -562,6 +605,22 @@ __global__ void attn_dkv_store_kernel(const AttnParams p) {
         __nv_bfloat16* out = (is_v ? p.dv : p.dk) + (int64_t)b * ss.stride_b + (int64_t)j * ss.stride_s + (int64_t)kvh * ss.stride_h + d;
         *reinterpret_cast<uint2*>(out) = make_uint2(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w));
     }
+}
+
+void launch_dkv_cluster(void (*kernel)(AttnParams), dim3 grid, int threads, int smem, cudaStream_t stream, const AttnParams& p) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = (unsigned)p.rep; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = dep_launch_enabled() ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, kernel, p);
 }
 
 // MFT_ATTN_SHAPE selects an alternative tile shape of the head_dim 256 kernels (tuning aid; 0 = default).
@@ -645,14 +704,17 @@ extern "C" int32_t mft_attn_bwd(const void* q, mft_strides_t sq, const void* k, 
     const int64_t rows = batch * n_heads * seq;
     const unsigned dblocks = (unsigned)((rows * 32 + 255) / 256);
     // dK / dV are collected in the caller's f32 scratch when it is given: by the tensor-memory kernel, or with one
-    // mma.sync CTA per query head when a KV group has several heads (more, shorter CTAs)
+    // mma.sync CTA per query head when a KV group has several heads (more, shorter CTAs; those of a short call as clusters,
+    // which do without it)
     const int shape = attn_shape_override();
     bool dkv_tc = false;
     // attn_dkv_store_kernel reads the scratch in 16-byte and writes dK / dV in 8-byte words; anywhere else than on such
     // addresses the kernel without scratch takes the call (its stores are 4 bytes)
     auto on = [](const void* q, uintptr_t bytes) { return reinterpret_cast<uintptr_t>(q) % bytes == 0; };
     if (!on(dkv_acc, 16) || !on(dk, 8) || !on(dv, 8)) p.dkv_acc = dkv_acc = nullptr;
-    if (dkv_acc != nullptr)
+    const bool cluster = dkv_acc != nullptr && attn_dkv_by_cluster(p, (int)hd);
+    if (cluster) p.dkv_acc = nullptr;            // without it the tensor-memory kernel declines
+    if (p.dkv_acc != nullptr)
         if (int32_t s = check_cuda(cudaMemsetAsync(dkv_acc, 0, (size_t)(2 * batch * seq * n_kv * hd) * sizeof(float), as_stream(stream)), "attention dkv memset")) return s;
     const bool split = dkv_acc != nullptr && p.rep > 1;
     dim3 gk((unsigned)((seq + 63) / 64), (unsigned)(split ? n_heads : n_kv), (unsigned)batch);
@@ -664,13 +726,14 @@ extern "C" int32_t mft_attn_bwd(const void* q, mft_strides_t sq, const void* k, 
         launch_dep(attn_bwd_dq_kernel<HD, BM, BN, ST>, dim3(gq), dim3(BM * 2), (size_t)(b1), as_stream(stream), p);                       \
         MFT_LAUNCH_CHECK("attn_bwd_dq");                                                                    \
     }
-#define DKV(HD, WN, SPLIT)                                                                                  \
+#define DKV(HD, WN, HEADS)                                                                                  \
     {                                                                                                       \
-        const int b2 = 6 * 64 * (HD + 8) * 2 + 2 * 64 * (64 + 8) * 2 + 4 * 64 * 4;                          \
-        if (int32_t s = set_smem(attn_bwd_dkv_kernel<HD, WN, SPLIT>, b2)) return s;                         \
-        launch_dep(attn_bwd_dkv_kernel<HD, WN, SPLIT>, dim3(gk), dim3(128 * WN), (size_t)(b2), as_stream(stream), p);                     \
+        const int b2 = dkv_smem_bytes(HD);                                                                  \
+        if (int32_t s = set_smem(attn_bwd_dkv_kernel<HD, WN, HEADS>, b2)) return s;                         \
+        if (HEADS == Heads::kCluster) launch_dkv_cluster(attn_bwd_dkv_kernel<HD, WN, HEADS>, gk, 128 * WN, b2, as_stream(stream), p);     \
+        else launch_dep(attn_bwd_dkv_kernel<HD, WN, HEADS>, dim3(gk), dim3(128 * WN), (size_t)(b2), as_stream(stream), p);                \
         MFT_LAUNCH_CHECK("attn_bwd_dkv");                                                                   \
-        if (SPLIT) {                                                                                        \
+        if (HEADS == Heads::kAtomic) {                                                                      \
             launch_dep(attn_dkv_store_kernel<HD>, dim3(148 * 8), dim3(256), (size_t)(0), as_stream(stream), p);                           \
             MFT_LAUNCH_CHECK("attn_dkv_store");                                                             \
         }                                                                                                   \
@@ -690,7 +753,9 @@ extern "C" int32_t mft_attn_bwd(const void* q, mft_strides_t sq, const void* k, 
         if (dkv_tc) {                                                                                       \
             launch_dep(attn_dkv_store_kernel<HD>, dim3(148 * 8), dim3(256), (size_t)(0), as_stream(stream), p);                           \
             MFT_LAUNCH_CHECK("attn_dkv_store");                                                             \
-        } else if (split) DKV(HD, WN, true) else DKV(HD, WN, false)                                         \
+        } else if (cluster) DKV(HD, WN, Heads::kCluster)                                                    \
+        else if (split) DKV(HD, WN, Heads::kAtomic)                                                         \
+        else DKV(HD, WN, Heads::kWhole)                                                                     \
     }
     if (hd == 64) { if (shape == 1) BWD(64, 1, 128, 64, 2) else BWD(64, 1, 64, 64, 2) }
     else if (hd == 128) BWD(128, 1, 64, 64, 2)

@@ -27,6 +27,8 @@ int32_t attn_dq_sm100(const AttnParams& p, int hd, bool compute_delta, cudaStrea
 // dK / dV of the backward pass ADDED into p.dkv_acc (f32 [2][batch, seq, n_kv, head_dim], zeroed by the caller);
 // needs p.dkv_acc and p.delta.
 int32_t attn_dkv_sm100(const AttnParams& p, int hd, cudaStream_t stream);
+// Short calls with grouped heads: dK / dV by clusters of mma.sync CTAs, in head order (attention.cu)
+bool attn_dkv_by_cluster(const AttnParams& p, int hd);
 
 // Any other head size (1..256): plain CUDA-core kernels, one CTA per row (attention_generic.cu).  The backward needs
 // p.delta as scratch; dK / dV are written directly (p.dkv_acc is not used).

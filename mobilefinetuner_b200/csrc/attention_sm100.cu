@@ -1045,18 +1045,29 @@ int32_t launch_dkv(const CUtensorMap& mq, const CUtensorMap& md, const CUtensorM
                               : launch_dkv_as<HD, true, false>(mq, md, mk, mv, p, seq, n_heads, batch, stream);
 }
 
+int attn_tc_mode() {
+    static const int v = [] { const char* e = std::getenv("MFT_ATTN_TC"); return e ? std::atoi(e) : 1; }();
+    return v;
+}
+
 // Where the backward kernels win over the mma.sync pair.  Microseconds mma.sync / tcgen05 of the whole backward pass, batch
-// 4 and 8:  head size 256, 4 heads:   64 tokens 28.6 / 25.5, 29.4 / 26.1;  128: 40.1 / 37.9, 41.6 / 40.2;  1000: 275 / 126, 433 / 211
+// 4 and 8:  head size 256, 4 / 1 heads:   64 tokens 28.6 / 25.5, 29.4 / 26.1;  128: 40.1 / 37.9, 41.6 / 40.2;  1000: 275 / 126, 433 / 211
 //   128, 8 heads:   128 tokens 29.4 / 30.5, 31.3 / 32.1;  160: 36.7 / 30.8, 48.1 / 33.7;  1000: 277 / 127, 476 / 211
 //   64, 14 / 2 heads:   160 tokens 33.2 / 31.4, 41.9 / 41.9;  200: 39.6 / 33.1, 54.2 / 44.0;  1000: 236 / 136, 403 / 224
 //   64, 12 / 12 heads:  160 tokens 25.8 / 26.0, 32.0 / 34.8;  200: 34.9 / 33.1, 44.8 / 45.0;  1000: 203 / 178, 345 / 295
-bool bwd_long_enough(int hd, int seq) { return hd == 256 || seq > (hd == 128 ? 128 : 192); }
+// At head size 256 a sequence of one 64-row tile leaves half of a tcgen05 CTA idle, and only one fits an SM: with more than
+// about a wave of them the mma.sync kernels win again (32 x 40 tokens, 4 / 1 heads 30.2 / 34.3; 32 x 64, 16 / 2 heads 95 / 121).
+constexpr int SHORT_GRID = 120;       // CTAs: the SMs that clusters of up to eight can fill, one CTA on each
+bool bwd_long_enough(const AttnParams& a, int hd) {
+    if (hd == 256) return a.seq > 64 || (int64_t)a.batch * a.n_heads <= SHORT_GRID;
+    return a.seq > (hd == 128 ? 128 : 192);
+}
 #define HD_DISPATCH(hd, CALL64, CALL128, CALL256) ((hd) == 64 ? (CALL64) : (hd) == 128 ? (CALL128) : (CALL256))
 
 }  // namespace
 
 int32_t attn_fwd_sm100(const AttnParams& a, int hd, cudaStream_t stream) {
-    static const int enabled = [] { const char* e = std::getenv("MFT_ATTN_TC"); return e ? std::atoi(e) : 1; }();
+    const int enabled = attn_tc_mode();
     if (!enabled || !tc_shape_ok(hd) || !device_status_word()) return MFT_ERR_UNSUPPORTED;
     if (!(a.scale > 0.f)) return MFT_ERR_UNSUPPORTED;      // the running maximum is taken before the scaling
     // A 128-query tile of this kernel against two 64-query CTAs of the mma.sync one: short sequences are bound by the
@@ -1090,10 +1101,21 @@ static int32_t box_map(CUtensorMap* map, const void* base, const AttnParams& a, 
                       : make_tmap_bf16(map, base, (int64_t)a.batch * a.seq, cols, ld, box_rows);
 }
 
+// Calls whose lengths are below the rule above, or of one 64-row tile at head size 256, in grids that fit the chip at once:
+// adding over the heads inside a cluster saves clearing, adding into and converting the f32 scratch, and gives the same bits
+// every time.  Microseconds with f32 atomics / cluster, whole backward:  head size 64, 14 / 2 heads:  4 x 40 16.4 / 15.2,
+// 8 x 128 30.0 / 28.0 (224 CTAs),  8 x 160 42.1 / 42.5 (336),  32 x 128 68.0 / 74.1;  128, 8 / 2 heads:  1 x 64 21.3 / 20.1,
+// 8 x 128 31.5 / 29.5 (128),  32 x 80 70 / 78 (512);  256, 4 / 1 heads (tcgen05 kernel / cluster):  1 x 40 23.2 / 23.6,
+// 1 x 64 25.5 / 26.4,  8 x 64 26.2 / 26.5;  16 / 2 heads:  8 x 40 33.7 / 37.9 (128 CTAs: 15 clusters of eight fit).
+bool attn_dkv_by_cluster(const AttnParams& a, int hd) {
+    if (attn_tc_mode() >= 2 || a.rep < 2 || a.rep > 8 || a.seq > (hd == 256 ? 64 : hd == 128 ? 128 : 192)) return false;
+    return (int64_t)((a.seq + 63) / 64) * a.n_heads * a.batch <= (hd == 64 ? 2 * num_sms() : SHORT_GRID);
+}
+
 int32_t attn_dq_sm100(const AttnParams& a, int hd, bool compute_delta, cudaStream_t stream) {
-    static const int enabled = [] { const char* e = std::getenv("MFT_ATTN_TC"); return e ? std::atoi(e) : 1; }();
+    const int enabled = attn_tc_mode();
     if (!enabled || !tc_shape_ok(hd) || !device_status_word()) return MFT_ERR_UNSUPPORTED;
-    if (!bwd_long_enough(hd, a.seq) && enabled < 2) return MFT_ERR_UNSUPPORTED;
+    if (!bwd_long_enough(a, hd) && enabled < 2) return MFT_ERR_UNSUPPORTED;
     if (compute_delta && hd != 256) return MFT_ERR_UNSUPPORTED;
     if (!aligned16(a.dq)) return MFT_ERR_UNSUPPORTED;
     if (!token_major(a.sq, a.seq) || !token_major(a.sk, a.seq) || !token_major(a.sv, a.seq) || !token_major(a.sdo, a.seq)) return MFT_ERR_UNSUPPORTED;
@@ -1121,9 +1143,9 @@ int32_t attn_dq_sm100(const AttnParams& a, int hd, bool compute_delta, cudaStrea
 }
 
 int32_t attn_dkv_sm100(const AttnParams& a, int hd, cudaStream_t stream) {
-    static const int enabled = [] { const char* e = std::getenv("MFT_ATTN_TC"); return e ? std::atoi(e) : 1; }();
+    const int enabled = attn_tc_mode();
     if (!enabled || !tc_shape_ok(hd) || !a.dkv_acc || !device_status_word()) return MFT_ERR_UNSUPPORTED;
-    if (!bwd_long_enough(hd, a.seq) && enabled < 2) return MFT_ERR_UNSUPPORTED;
+    if (!bwd_long_enough(a, hd) && enabled < 2) return MFT_ERR_UNSUPPORTED;
     if (!token_major(a.sq, a.seq) || !token_major(a.sk, a.seq) || !token_major(a.sv, a.seq) || !token_major(a.sdo, a.seq)) return MFT_ERR_UNSUPPORTED;
     if (a.sq.stride_h % 8 || a.sk.stride_h % 8 || a.sv.stride_h % 8 || a.sdo.stride_h % 8) return MFT_ERR_UNSUPPORTED;
     if ((int64_t)a.batch * a.seq >= (1ll << 31) || 2 * a.n_heads > 65535) return MFT_ERR_UNSUPPORTED;

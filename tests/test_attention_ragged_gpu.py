@@ -81,3 +81,29 @@ def test_outputs_off_16_bytes(hd, heads, kv, seq, shift):
         assert (x.float() - r).norm() <= 2 ** -7 * r.norm(), name       # as above
     for buf in (o_buf, dq_buf, dk_buf, dv_buf):
         assert bool(buf[:shift].isnan().all()) and bool(buf[buf.numel() - 8 + shift:].isnan().all())
+
+
+# short calls with grouped heads: dK / dV are added over the heads of a group inside a cluster, in head order.  Group sizes up
+# to eight (nine goes another way), one and several 64-key tiles, both sides of the grid limits and of the lengths
+@pytest.mark.parametrize("hd,heads,kv,seq,window,batch", [
+    (64, 14, 2, 2, 0, 1), (64, 14, 2, 65, 0, 2), (64, 8, 1, 192, 70, 3), (64, 6, 2, 130, 0, 8), (64, 9, 1, 63, 0, 2), (64, 4, 2, 64, 0, 80),
+    (128, 8, 2, 100, 0, 1), (128, 6, 2, 128, 33, 2), (128, 8, 1, 64, 0, 16), (256, 4, 1, 40, 0, 2), (256, 4, 1, 64, 20, 30), (256, 8, 1, 33, 0, 1),
+    (256, 4, 1, 64, 0, 31), (256, 6, 2, 17, 0, 3)])
+def test_short_grouped_backward(hd, heads, kv, seq, window, batch):
+    from mobilefinetuner_b200 import ops as O
+    g = torch.Generator(device="cuda").manual_seed(seq + batch)
+
+    def rnd(n):
+        return torch.randn(batch, seq, n, hd, device="cuda", generator=g).bfloat16().permute(0, 2, 1, 3)
+    q, k, v, d_o = rnd(heads), rnd(kv), rnd(kv), rnd(heads)
+    scale = hd ** -0.5
+    o, lse = O.attention_fwd(q, k, v, scale, window)
+    got = O.attention_bwd(q, k, v, o, d_o, lse, scale, window)
+    ref = _reference(q, k, v, d_o, scale, window)
+    for name, a, b in zip(("dq", "dk", "dv"), got, ref[2:]):
+        assert (a.float() - b).norm() <= 2 ** -7 * b.norm(), name       # as above
+    tiles = (seq + 63) // 64 * heads * batch
+    if heads // kv <= 8 and tiles <= (296 if hd == 64 else 120):        # by clusters (148 SMs): the same bits every time
+        for _ in range(10):
+            again = O.attention_bwd(q, k, v, o, d_o, lse, scale, window)
+            assert all(torch.equal(a, b) for a, b in zip(got, again))
