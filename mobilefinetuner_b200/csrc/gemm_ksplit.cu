@@ -8,9 +8,9 @@
 // the columns (8-column groups dealt to the ranks; the pipeline stages serve as the exchange area), and every owner adds
 // its S slices in rank order and stores bf16.  No workspace, no atomics, one launch, and the result does not depend on timing.
 //
-// Bound by shared-memory traffic in the K loop (0.30 us per k-block of a 128 x 128 tile: 32 KB written by the TMA unit, 32
-// read by the MMAs) and by about 3 us for the two cluster barriers and the exchange.  ksplit_plan() weighs that against the
-// tile counts of the other kernels.  Measured per launch (20 in a graph, operands rotating over more than the L2):
+// A k-block of a 128 x 128 tile takes 0.30 us, about 570 clocks for its 32 KB: 57 bytes a clock into each SM, where a copy-only
+// kernel brings in 72 (microbench tma).  The two cluster barriers and the exchange add about 3 us.  ksplit_plan() weighs that
+// against the tile counts of the other kernels.  Measured per launch (20 in a graph, operands rotating over more than the L2):
 //     512 x 1152 x 13824   67.3 -> 27.9 us        512 x 768 x 3072   19.8 -> 11.3 us
 //     512 x 1152 x  6912   37.2 -> 18.6           512 x 896 x 4864   28.0 -> 13.7
 //     512 x   32 x 13824   55.0 -> 12.9          4096 x  16 x 6912   30.2 -> 15.2
