@@ -323,7 +323,7 @@ int32_t mft_glu_linear_bwd(int32_t kind, const void* dy_bf16, int64_t lddy, cons
  * head_dim 64 / 128 / 256 with token-major tensors (stride_b == seq *
  * stride_s) runs on tensor-memory (tcgen05) kernels, except for short
  * sequences, where the mma.sync kernels are the faster ones (up to 384 / 128 /
- * 256 tokens forward, 192 / 128 / 64 backward); other shapes of those head sizes on mma.sync kernels,
+ * 256 tokens forward, 192 / 128 / 64 backward, a little more in large grids); other shapes of those head sizes on mma.sync kernels,
  * any other even head_dim <= 256 on generic kernels, all with the same results
  * to bf16 rounding.  MFT_ATTN_TC=0 in the environment selects the mma.sync
  * kernels everywhere, MFT_ATTN_TC=2 the tensor-memory kernels at every shape

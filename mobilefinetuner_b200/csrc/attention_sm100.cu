@@ -1075,8 +1075,11 @@ int32_t attn_fwd_sm100(const AttnParams& a, int hd, cudaStream_t stream) {
     // tcgen05 (batch 4 and 8):  head size 256, 4 heads:   256 tokens 17.9 / 18.0, 18.0 / 18.1;  300: 20.5 / 18.1, 25.9 / 18.4
     //   128, 8 heads:   128 tokens 8.0 / 9.6, 8.1 / 10.0;  160: 9.7 / 9.7, 12.8 / 10.0
     //   64, 14 heads:   384 tokens 18.2 / 17.1, 24.0 / 25.6;  437: 19.6 / 18.2, 30.6 / 29.8
-    // and 113 / 49, 110 / 57, 100 / 66 at 8 x 1000.  MFT_ATTN_TC=2 forces it.
-    if (a.seq <= (hd == 256 ? 256 : hd == 128 ? 128 : 384) && enabled < 2) return MFT_ERR_UNSUPPORTED;
+    // and 113 / 49, 110 / 57, 100 / 66 at 8 x 1000.  At batch 1 no length got slower by the same rule.  More than a wave of
+    // these CTAs at head size 128, three 64-query tiles against two of 128:  16 x 160, 8 heads 17.4 / 19.1,  64 x 192 52.4 / 61.0,
+    // but  64 x 193 75.2 / 63.9 and  8 x 160 13.3 / 10.6 (128 CTAs).  MFT_ATTN_TC=2 forces it.
+    const bool crowded = (int64_t)((a.seq + BM - 1) / BM) * a.n_heads * a.batch > num_sms();
+    if (a.seq <= (hd == 256 ? 256 : hd == 128 ? (crowded ? 192 : 128) : 384) && enabled < 2) return MFT_ERR_UNSUPPORTED;
     if (!token_major(a.sq, a.seq) || !token_major(a.sk, a.seq) || !token_major(a.sv, a.seq)) return MFT_ERR_UNSUPPORTED;
     if (a.sq.stride_h % 8 || a.sk.stride_h % 8 || a.sv.stride_h % 8 || a.so.stride_s % 8 || a.so.stride_h % 8 || a.so.stride_b % 8) return MFT_ERR_UNSUPPORTED;
     if (!aligned16(a.out)) return MFT_ERR_UNSUPPORTED;
@@ -1117,6 +1120,11 @@ int32_t attn_dq_sm100(const AttnParams& a, int hd, bool compute_delta, cudaStrea
     if (!enabled || !tc_shape_ok(hd) || !device_status_word()) return MFT_ERR_UNSUPPORTED;
     if (!bwd_long_enough(a, hd) && enabled < 2) return MFT_ERR_UNSUPPORTED;
     if (compute_delta && hd != 256) return MFT_ERR_UNSUPPORTED;
+    // Head size 64 without grouped heads, where this is the only tensor-memory kernel of the pass: with more CTAs than the chip
+    // holds (two per SM) the mma.sync one wins up to 320 tokens.  12 heads, microseconds mma.sync / tcgen05 of the pass:
+    // 16 x 193 70.5 / 71.9,  16 x 257 95.6 / 103.6,  64 x 320 338 / 350,  16 x 321 126.2 / 124.9;  8 x 257 58.0 / 57.3 (288 CTAs)
+    if (hd == 64 && a.rep == 1 && a.seq <= 320 && (int64_t)((a.seq + BM - 1) / BM) * a.n_heads * a.batch > 2 * num_sms() && enabled < 2)
+        return MFT_ERR_UNSUPPORTED;
     if (!aligned16(a.dq)) return MFT_ERR_UNSUPPORTED;
     if (!token_major(a.sq, a.seq) || !token_major(a.sk, a.seq) || !token_major(a.sv, a.seq) || !token_major(a.sdo, a.seq)) return MFT_ERR_UNSUPPORTED;
     if (a.sq.stride_h % 8 || a.sk.stride_h % 8 || a.sv.stride_h % 8 || a.sdo.stride_h % 8) return MFT_ERR_UNSUPPORTED;
